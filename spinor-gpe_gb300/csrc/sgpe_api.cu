@@ -72,6 +72,14 @@ struct SepOps {
   // of the components differ by a constant (pb_1 = kappa pb_0)
   DevField m[4], dg[2], mb;
   bool fused_c = false, fused_d = false, mb_real = false;
+  // complex128 plans: the same tables as split fixed-point factors
+  // (sgpe_fx.cuh), times 2^-exponent; not made when a table holds a value
+  // that is not finite
+  void* fky[2] = {nullptr, nullptr};
+  void* fm = nullptr;    // m[0..3] one after the other
+  void* fdg = nullptr;   // dg[0..1]
+  int fke[2] = {0, 0}, fme = 0, fdge = 0;
+  bool fx_kin = false, fx_c = false, fx_d = false;
 };
 
 // True when every value of the field has a zero imaginary part.
@@ -149,10 +157,11 @@ struct sgpe_plan {
   double* fin = nullptr;     // their sums (3 doubles) and the pass's arrival
   unsigned* count = nullptr; // counter, behind the partials in `part`
   // the last column block forms the sums once and row blocks read them
-  // (double-float plans, where every row block re-summing the partials in
-  // double-float arithmetic cost ~10% of the row pass); complex64 and
-  // complex128 row blocks sum the partials themselves while their other
-  // warps transform, which costs less than a serial tail on the column pass
+  // (double-float and complex128 plans, where every row block re-summing the
+  // partials cost ~10% of the double-float row pass and would be the
+  // fixed-point row pass's longest FP64 chain); complex64 row blocks sum the
+  // partials themselves while their other warps transform, which costs less
+  // than a serial tail on the column pass
   bool final_sums = false;
   int ntile = 0;             // column tiles of the current kernels
   int ntile_fp32 = 0;        // ... of the FP32 DFT kernels
@@ -162,6 +171,9 @@ struct sgpe_plan {
   uint32_t* tcb = nullptr;   // their B fragments (device)
   void* tw_x = nullptr;
   void* tw_y = nullptr;
+  // twiddles of the fixed-point passes (complex128 plans)
+  void* twf_x = nullptr;
+  void* twf_y = nullptr;
   // complex128 twiddle tables of a double-float plan, for its complex128
   // transforms (sgpe_fft2, the energy functional); made on first use
   void* tw64_x = nullptr;
@@ -208,6 +220,7 @@ struct BatchGroup {
   std::vector<int> members;  // indices into sgpe_batch::plans
   int nx = 0, ny = 0, bits = 0;
   int row_shape = 0, col_shape = 0;  // the members' kernel shapes (equal)
+  bool fx = false;           // complex128 in fixed point (all members)
   void* col_args = nullptr;  // device ColArgs[3][G]: (0 -> 0), (0 -> 1), (1 -> 0)
   void* row_args = nullptr;  // device RowArgs[2][G]: sub-steps 0, 1
   cudaStream_t stream = nullptr;
@@ -295,6 +308,64 @@ template <typename R> void* upload_twiddles(int n, int e, cudaError_t* err) {
   return d;
 }
 
+// Split fixed-point factor (fx_cmul) of two 64-bit integers.
+int4 fx_entry(long long re, long long im) {
+  auto split = [](long long w, int* h, int* l) {
+    *l = int(uint32_t(uint64_t(w)));
+    if (*l == INT32_MIN) ++*l;  // the kernels negate low words
+    *h = int((w - *l) >> 32);
+  };
+  int4 r;
+  split(re, &r.x, &r.y);
+  split(im, &r.z, &r.w);
+  return r;
+}
+
+int upload_int4(const std::vector<int4>& h, void** out, std::vector<void*>* allocs, const char* name) {
+  cudaError_t e = cudaMalloc(out, sizeof(int4) * h.size());
+  if (e != cudaSuccess) return fail(SGPE_ERR_OOM, std::string(name) + ": " + cudaGetErrorString(e));
+  if (allocs != nullptr) allocs->push_back(*out);
+  e = cudaMemcpy(*out, h.data(), sizeof(int4) * h.size(), cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? SGPE_OK : cuda_fail(e, name);
+}
+
+// Twiddle table of an (n, e) transform in fixed point: the entries of
+// upload_twiddles times 2^(64 - fx_stage_bits) (sgpe_fx.cuh).  The roots of
+// order n are products of two short tables evaluated in extended precision,
+// rounded at 2^-62 (evaluating every root so took 2 ms a plan).
+int upload_twiddles_fx(int n, int e, void** out) {
+  struct Root {
+    long long re, im;  // times 2^62
+  };
+  constexpr int kFine = 64;
+  const long double two_pi = 6.283185307179586476925286766559005768L;
+  auto root = [&](int m) {
+    const long double a = two_pi * (long double)m / (long double)n;
+    return Root{llrintl(ldexpl(cosl(a), 62)), llrintl(ldexpl(-sinl(a), 62))};
+  };
+  std::vector<Root> fine(kFine), coarse((n + kFine - 1) / kFine);
+  for (int m = 0; m < kFine; ++m) fine[m] = root(m);
+  for (size_t m = 0; m < coarse.size(); ++m) coarse[m] = root(int(m) * kFine);
+  auto scaled = [](__int128 v, int bits) { return (long long)((v + ((__int128)1 << (bits - 1))) >> bits); };
+  std::vector<int4> h;
+  for (int ns = 1; ns < n;) {
+    const int rs = sgpe::stage_radix(n, e, ns);
+    const int len = ns * rs;
+    const int down = 60 + sgpe::fx_stage_bits(rs, len == n);  // 2^124 -> 2^(64 - bits)
+    for (int r = 1; r < rs; ++r)
+      for (int k = 0; k < ns; ++k) {
+        const int m = int(((long long)k * r) % len) * (n / len);
+        const Root &a = fine[m % kFine], &b = coarse[m / kFine];
+        const __int128 re = (__int128)a.re * b.re - (__int128)a.im * b.im;
+        const __int128 im = (__int128)a.re * b.im + (__int128)a.im * b.re;
+        h.push_back(fx_entry(scaled(re, down), scaled(im, down)));
+      }
+    ns = len;
+  }
+  if (h.empty()) h.push_back(fx_entry(1ll << 62, 0));
+  return upload_int4(h, out, nullptr, "fixed-point twiddles");
+}
+
 // Default kernel shape of a pass (axis 0: rows along x, 1: columns along y)
 // for a side n, from single-solve step times of square grids measured on
 // GB300 with sgpe_autotune (real and imaginary time ranked alike): fewer
@@ -310,7 +381,7 @@ int default_shape(int bits, int axis, int n) {
     int n, row, col;
   };
   static const Entry f32[] = {{32, 2, 1}, {64, 2, 2}, {128, 2, 1}, {256, 2, 0}, {512, 1, 0}};
-  static const Entry f64[] = {{32, 2, 1}, {64, 2, 1}, {128, 2, 1}, {256, 2, 0}, {512, 0, 0}};
+  static const Entry f64[] = {{32, 2, 1}, {64, 2, 1}, {128, 2, 1}, {256, 2, 2}, {512, 0, 0}};
   if (bits == SGPE_DTYPE_DF) return 0;
   for (const Entry& x : (bits == 64 ? f32 : f64))
     if (x.n == n) return axis == 0 ? x.row : x.col;
@@ -466,6 +537,31 @@ HostField host_field(const sgpe_field& f) {
   return h;
 }
 
+// Smallest e with every |value| of the fields at most 2^e (to rounding);
+// false when a value is not finite.
+bool fx_exponent(std::initializer_list<const HostField*> fields, int* e) {
+  double most = 0.0;
+  for (const HostField* f : fields)
+    for (size_t i = 0; i < f->v.size(); i += 2) {
+      const double m = std::hypot(f->v[i], f->v[i + 1]);
+      if (!std::isfinite(m)) return false;
+      most = std::max(most, m);
+    }
+  *e = 0;
+  if (most > 0.0) std::frexp(most * (1.0 - 1e-9), e);
+  return true;
+}
+
+// Tables of equal length as split fixed-point factors, value 2^(62 - e), one
+// after the other.
+int upload_fx(std::initializer_list<const HostField*> fields, int e, void** out, std::vector<void*>* allocs) {
+  std::vector<int4> h;
+  for (const HostField* f : fields)
+    for (size_t i = 0; i < f->v.size(); i += 2)
+      h.push_back(fx_entry(std::llrint(std::ldexp(f->v[i], 62 - e)), std::llrint(std::ldexp(f->v[i + 1], 62 - e))));
+  return upload_int4(h, out, allocs, "fixed-point table");
+}
+
 // Kinetic part of SepOps from the FP64 factors of each component.
 int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2], SepOps* so,
                   std::vector<void*>* allocs) {
@@ -478,6 +574,14 @@ int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2]
     if (rc != SGPE_OK) return rc;
   }
   so->kin = true;
+  if (p->bits != 128) return SGPE_OK;
+  for (int c = 0; c < 2; ++c) {
+    int ex = 0;
+    if (!fx_exponent({&x[c]}, &ex) || !fx_exponent({&y[c]}, &so->fke[c])) return SGPE_OK;
+    const int rc = upload_fx({&y[c]}, so->fke[c], &so->fky[c], allocs);
+    if (rc != SGPE_OK) return rc;
+  }
+  so->fx_kin = true;
   return SGPE_OK;
 }
 
@@ -533,10 +637,21 @@ int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2]
   if (rc != SGPE_OK) return rc;
   so->mb_real = imag_zero(py[0]);
   so->fused_d = true;
+  const bool fx = p->bits == 128;
+  if (fx && fx_exponent({&dg[0], &dg[1]}, &so->fdge)) {
+    rc = upload_fx({&dg[0], &dg[1]}, so->fdge, &so->fdg, allocs);
+    if (rc != SGPE_OK) return rc;
+    so->fx_d = true;
+  }
   if (s01 != nullptr) {
     for (int k = 0; k < 4 && rc == SGPE_OK; ++k) rc = upload_host_field(p, m[k], &so->m[k], allocs);
     if (rc != SGPE_OK) return rc;
     so->fused_c = true;
+    if (fx && fx_exponent({&m[0], &m[1], &m[2], &m[3]}, &so->fme)) {
+      rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, so->fme, &so->fm, allocs);
+      if (rc != SGPE_OK) return rc;
+      so->fx_c = true;
+    }
   }
   return SGPE_OK;
 }
@@ -661,6 +776,42 @@ template <typename R> sgpe::RealOp<R> real_op(const SubOps& so, int coupling) {
 template <typename R> sgpe::Cx<R>* st(void* p) { return static_cast<sgpe::Cx<R>*>(p); }
 template <typename R> const sgpe::Cx<R>* cst(const void* p) { return static_cast<const sgpe::Cx<R>*>(p); }
 
+// Fixed-point column operands of the kinetic factors applied (one or two
+// sets); without tables for one of them the FP64 kernels run.
+template <typename R> void col_fx(const sgpe_plan*, std::initializer_list<const SepOps*>, sgpe::ColArgs<R>*) {}
+template <>
+void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops, sgpe::ColArgs<double>* a) {
+  int i = 0;
+  for (const SepOps* s : ops) {
+    if (!s->fx_kin) return;
+    for (int c = 0; c < 2; ++c) {
+      a->kb[i][c] = static_cast<const int4*>(s->fky[c]);
+      a->ke[i][c] = s->fke[c];
+    }
+    ++i;
+  }
+  a->twf = static_cast<const int4*>(p->twf_y);
+}
+
+// Whether the row pass of sub-step `so` can run in fixed point: separable
+// operators with finite tables, an interaction factor that is a phase or
+// never above one (the point-wise results have no headroom to grow into),
+// and the column pass's final sums.
+bool row_fx_ok(const sgpe_plan* p, const SubOps& so) {
+  if (p->bits != 128 || !p->final_sums || !fused_sep(so, p->coupling)) return false;
+  if (!(p->coupling ? so.sep.fx_c : so.sep.fx_d)) return false;
+  if (so.zr == 0.0) return true;
+  return so.zi == 0.0 && so.zr * p->g[0] <= 0.0 && so.zr * p->g[1] <= 0.0 && so.zr * p->g[2] <= 0.0;
+}
+template <typename R> void row_fx(const sgpe_plan*, const SubOps&, sgpe::RowArgs<R>*) {}
+template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowArgs<double>* a) {
+  if (!row_fx_ok(p, so)) return;
+  const int4* m = static_cast<const int4*>(p->coupling ? so.sep.fm : so.sep.fdg);
+  for (int k = 0; k < 4; ++k) a->mf[k] = m + (p->coupling ? k : k / 2) * p->nx;
+  a->me = p->coupling ? so.sep.fme : so.sep.fdge;
+  a->twf = static_cast<const int4*>(p->twf_x);
+}
+
 // Column pass over the state (in place) ending a sub-step and starting `sub`.
 // want_u: the populations of the state entering the pass are needed, so the
 // two kinetic half steps are applied separately (sum after the first).
@@ -686,14 +837,17 @@ template <typename R> bool col_step_args(sgpe_plan* p, int sub, bool want_u, sgp
   if (p->form != kMixed) {
     a.nk = 1;
     a.k1 = kin_op<R>(p->sub[sub]);
+    col_fx<R>(p, {&p->sub[sub].sep}, &a);
   } else if (want_u) {
     a.nk = 2;
     a.k1 = kin_op<R>(p->sub[p->prev_sub]);
     a.k2 = kin_op<R>(p->sub[sub]);
+    col_fx<R>(p, {&p->sub[p->prev_sub].sep, &p->sub[sub].sep}, &a);
   } else {
     if (ensure_pair(p, p->prev_sub, sub) != SGPE_OK) return false;
     a.nk = 1;
     a.k1 = kin_pair<R>(p->pair[p->prev_sub][sub]);
+    col_fx<R>(p, {&p->pair[p->prev_sub][sub].sep}, &a);
   }
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
@@ -731,6 +885,7 @@ template <typename R> sgpe::RowArgs<R> row_step_args(sgpe_plan* p, int sub, doub
   a.g_ud = R(p->g[2]);
   a.coupling = p->coupling;
   a.op = real_op<R>(p->sub[sub], p->coupling);
+  row_fx<R>(p, p->sub[sub], &a);
   a.pops = pops;
   a.atom_num = p->atom_num;
   return a;
@@ -875,6 +1030,7 @@ template <typename R> int store(sgpe_plan* p, void* o0, void* o1, double* pops, 
   a.k1 = kin_op<R>(p->sub[p->prev_sub]);
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
+  col_fx<R>(p, {&p->sub[p->prev_sub].sep}, &a);
   cudaError_t e = sgpe::launch_col<R>(a, p->ny, s);
   if (e != cudaSuccess) return cuda_fail(e, "store (column pass)");
   sgpe::ScaleArgs<R> sa{};
@@ -948,6 +1104,12 @@ template <typename R> int fft2(sgpe_plan* p, const void* i0, const void* i1, voi
   c.shape = own ? p->col_shape : 0;
   c.nx = p->nx;
   c.scale = R(1);
+  if constexpr (std::is_same<R, double>::value) {
+    if (own) {
+      r.twf = static_cast<const int4*>(p->twf_x);
+      c.twf = static_cast<const int4*>(p->twf_y);
+    }
+  }
   cudaError_t e;
   if (!inverse) {
     r.in[0] = cst<R>(i0);
@@ -1137,21 +1299,27 @@ template <typename R> int apply_shapes(sgpe_plan* p, int rs, int cs) {
   if (rs != p->row_shape) tx = upload_twiddles<R>(p->nx, sgpe::row_points_per_thread<R>(p->nx, rs), &e);
   if (e == cudaSuccess && cs != p->col_shape)
     ty = upload_twiddles<R>(p->ny, sgpe::col_points_per_thread<R>(p->ny, cs), &e);
+  void* fx = nullptr;
+  void* fy = nullptr;
+  if (p->bits == 128) {
+    if (e == cudaSuccess && tx && upload_twiddles_fx(p->nx, sgpe::row_points_per_thread<R>(p->nx, rs), &fx) != SGPE_OK)
+      e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess && ty && upload_twiddles_fx(p->ny, sgpe::col_points_per_thread<R>(p->ny, cs), &fy) != SGPE_OK)
+      e = cudaErrorMemoryAllocation;
+  }
   if (e != cudaSuccess) {
-    if (tx) cudaFree(tx);
-    if (ty) cudaFree(ty);
+    for (void* t : {tx, ty, fx, fy})
+      if (t) cudaFree(t);
     return fail(SGPE_ERR_OOM, std::string("twiddle tables: ") + cudaGetErrorString(e));
   }
   drop_graphs(p);
   // cudaFree waits for launches still reading the old tables
-  if (tx) {
-    cudaFree(p->tw_x);
-    p->tw_x = tx;
-  }
-  if (ty) {
-    cudaFree(p->tw_y);
-    p->tw_y = ty;
-  }
+  const struct { void** own; void* made; } tables[] = {{&p->tw_x, tx}, {&p->tw_y, ty}, {&p->twf_x, fx}, {&p->twf_y, fy}};
+  for (const auto& t : tables)
+    if (t.made) {
+      cudaFree(*t.own);
+      *t.own = t.made;
+    }
   p->row_shape = rs;
   p->col_shape = cs;
   p->ntile_fp32 = p->nx / cols;
@@ -1217,7 +1385,7 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
   p->graphs_enabled = std::getenv("SGPE_DISABLE_GRAPHS") == nullptr;
   // SGPE_FINAL_SUMS=0/1 overrides the precision's choice (measurements)
   const char* fs = std::getenv("SGPE_FINAL_SUMS");
-  p->final_sums = fs != nullptr ? fs[0] == '1' : dtype_bits == SGPE_DTYPE_DF;
+  p->final_sums = fs != nullptr ? fs[0] == '1' : dtype_bits != 64;
   p->row_shape = default_shape(dtype_bits, 0, nx);
   p->col_shape = default_shape(dtype_bits, 1, ny);
   int cols = by_prec(dtype_bits, [&](auto t) { return sgpe::col_tile_width<decltype(t)>(ny, p->col_shape); });
@@ -1250,6 +1418,10 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
       return 0;
     });
   }
+  if (e == cudaSuccess && dtype_bits == 128 &&
+      (upload_twiddles_fx(nx, sgpe::row_points_per_thread<double>(nx, p->row_shape), &p->twf_x) != SGPE_OK ||
+       upload_twiddles_fx(ny, sgpe::col_points_per_thread<double>(ny, p->col_shape), &p->twf_y) != SGPE_OK))
+    e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->derr), sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(p->derr, 0, sizeof(int));
   if (e != cudaSuccess) {
@@ -1274,6 +1446,8 @@ int sgpe_plan_destroy(sgpe_plan* p) {
   if (p->part) cudaFree(p->part);
   if (p->tw_x) cudaFree(p->tw_x);
   if (p->tw_y) cudaFree(p->tw_y);
+  if (p->twf_x) cudaFree(p->twf_x);
+  if (p->twf_y) cudaFree(p->twf_y);
   if (p->tw64_x) cudaFree(p->tw64_x);
   if (p->tw64_y) cudaFree(p->tw64_y);
   free_sub(p->sub[0]);
@@ -1964,7 +2138,16 @@ template <typename R> int launch_group_steps(const BatchGroup& g, int steps) {
   const int cv[3] = {0, 1, 2}, rs[3] = {0, 1, 0};
   for (int k = 0; k < steps; ++k)
     for (int t = 0; t < 3; ++t) {
-      cudaError_t e = sgpe::launch_col_grouped<R>(col + cv[t] * G, g.col_shape, G, g.nx, g.ny, g.stream);
+      cudaError_t e = cudaSuccess;
+      if constexpr (std::is_same<R, double>::value) {
+        if (g.fx) {
+          e = sgpe::launch_col_fx(col + cv[t] * G, g.col_shape, G, g.nx, g.ny, g.stream);
+          if (e == cudaSuccess) e = sgpe::launch_row_fx(row + rs[t] * G, g.row_shape, G, g.nx, g.ny, g.stream);
+          if (e != cudaSuccess) return cuda_fail(e, "batch grouped pass");
+          continue;
+        }
+      }
+      e = sgpe::launch_col_grouped<R>(col + cv[t] * G, g.col_shape, G, g.nx, g.ny, g.stream);
       if (e == cudaSuccess)
         e = sgpe::launch_row_grouped<R>(row + rs[t] * G, g.row_shape, G, g.nx, g.ny, g.stream);
       if (e != cudaSuccess) return cuda_fail(e, "batch grouped pass");
@@ -1987,8 +2170,17 @@ void build_groups(sgpe_batch* b) {
         if (!fused_sep(q->sub[sub], q->coupling)) return false;
       return true;
     };
-    if (!b->grouping || !sep(p)) continue;
+    // the grouped passes are all fixed point or all FP64, as the plans' own
+    // are; a plan that mixes the two stays alone
+    auto fx = [](const sgpe_plan* q) {
+      int n = 0;
+      for (int sub = 0; sub < 2; ++sub) n += row_fx_ok(q, q->sub[sub]) ? 1 : 0;
+      for (int v = 0; v < 3; ++v) n += q->pair[v == 2][v == 1].sep.fx_kin ? 1 : 0;
+      return n == 5 ? 1 : n == 0 ? 0 : -1;
+    };
+    if (!b->grouping || !sep(p) || fx(p) < 0) continue;
     BatchGroup g;
+    g.fx = fx(p) == 1;
     g.nx = p->nx;
     g.ny = p->ny;
     g.bits = p->bits;
@@ -1997,7 +2189,7 @@ void build_groups(sgpe_batch* b) {
     for (size_t k = i; k < b->plans.size(); ++k) {
       const sgpe_plan* q = b->plans[k];
       if (!taken[k] && q->nx == p->nx && q->ny == p->ny && q->bits == p->bits && q->row_shape == p->row_shape &&
-          q->col_shape == p->col_shape && sep(q))
+          q->col_shape == p->col_shape && sep(q) && fx(q) == fx(p))
         g.members.push_back(int(k));
     }
     if (g.members.size() < 2) continue;

@@ -45,16 +45,19 @@
 #include <type_traits>
 
 #include "sgpe_df.cuh"
+#include "sgpe_fx.cuh"
 #include "sgpe_tc.cuh"
 
 namespace sgpe {
 
 // Complex element type of each precision: complex64 (float2), complex128
-// (double2) and double-float (DFC, FP32 head + tail pairs).
+// (double2) and double-float (DFC, FP32 head + tail pairs); fx_t is the
+// fixed-point form complex128 lines take inside a transform (sgpe_fx.cuh).
 template <typename R> struct CxT;
 template <> struct CxT<float> { using type = float2; };
 template <> struct CxT<double> { using type = double2; };
 template <> struct CxT<DF> { using type = DFC; };
+template <> struct CxT<fx_t> { using type = FxC; };
 template <typename R> using Cx = typename CxT<R>::type;
 
 // conversion between a storage complex type CS and a compute type C
@@ -74,6 +77,7 @@ template <typename R> struct TwT { using type = Cx<R>; };
 template <> struct TwT<float> { using type = float4; };
 #endif
 template <> struct TwT<DF> { using type = float4; };
+template <> struct TwT<fx_t> { using type = int4; };  // split factors (fx_cmul)
 template <typename R> using TwE = typename TwT<R>::type;
 
 __device__ __forceinline__ float fmadd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -149,6 +153,39 @@ template <class C> __device__ __forceinline__ decltype(C::x) cabs2(C a) { return
 template <int DIR, class C> __device__ __forceinline__ C crot(C a) {
   return DIR < 0 ? cmake<C>(a.y, -a.x) : cmake<C>(-a.y, a.x);
 }
+// fixed point: factors from the stage's table carry its 2^-bits(R)
+template <int DIR> __device__ __forceinline__ FxC tw_mul(FxC a, int4 w) { return fx_cmul<(DIR > 0)>(a, w); }
+// cos(pi/12), sqrt(3)/2, sqrt(1/2), sin(pi/12), cos(pi/8), sin(pi/8) times a
+// (64-bit constants relative to one or zero, fx_mulc)
+__device__ __forceinline__ fx_t fx_cos15(fx_t a) { return fx_mulc<1, -628557561968679382ll>(a); }
+__device__ __forceinline__ fx_t fx_cos30(fx_t a) { return fx_mulc<1, -2471395088767036514ll>(a); }
+__device__ __forceinline__ fx_t fx_cos45(fx_t a) { return fx_mulc<1, -5402926248376769404ll>(a); }
+__device__ __forceinline__ fx_t fx_sin15(fx_t a) { return fx_mulc<0, 4774368686408090022ll>(a); }
+__device__ __forceinline__ fx_t fx_cos22(fx_t a) { return fx_mulc<1, -1404174782535421627ll>(a); }
+__device__ __forceinline__ fx_t fx_sin22(fx_t a) { return fx_mulc<0, 7059263338087549767ll>(a); }
+// a exp(DIR 2 pi i QUAD / 4), exact
+template <int DIR, int QUAD> __device__ __forceinline__ FxC fx_quad(FxC a) {
+  if constexpr (QUAD == 0) return a;
+  else if constexpr (QUAD == 1) return crot<DIR>(a);
+  else if constexpr (QUAD == 2) return FxC{-a.x, -a.y};
+  else return crot<-DIR>(a);
+}
+// a exp(DIR 2 pi i M / 48), M = 0..11 a multiple of 2 or 3 (the roots of
+// order 16 and 24 of the first quadrant)
+template <int DIR, int M> __device__ __forceinline__ FxC fx_root(FxC a) {
+  if constexpr (M == 0) return a;
+  else if constexpr (M == 6) return FxC{fx_cos45(a.x - sgn<DIR>(a.y)), fx_cos45(a.y + sgn<DIR>(a.x))};
+  else if constexpr (M == 2) return FxC{fx_cos15(a.x) - sgn<DIR>(fx_sin15(a.y)), fx_cos15(a.y) + sgn<DIR>(fx_sin15(a.x))};
+  else if constexpr (M == 3) return FxC{fx_cos22(a.x) - sgn<DIR>(fx_sin22(a.y)), fx_cos22(a.y) + sgn<DIR>(fx_sin22(a.x))};
+  else if constexpr (M == 4) return FxC{fx_cos30(a.x) - sgn<DIR>(a.y >> 1), fx_cos30(a.y) + sgn<DIR>(a.x >> 1)};
+  else if constexpr (M == 8) return FxC{(a.x >> 1) - sgn<DIR>(fx_cos30(a.y)), (a.y >> 1) + sgn<DIR>(fx_cos30(a.x))};
+  else if constexpr (M == 9) return FxC{fx_sin22(a.x) - sgn<DIR>(fx_cos22(a.y)), fx_sin22(a.y) + sgn<DIR>(fx_cos22(a.x))};
+  else {
+    static_assert(M == 10, "no constant root");
+    return FxC{fx_sin15(a.x) - sgn<DIR>(fx_cos15(a.y)), fx_sin15(a.y) + sgn<DIR>(fx_cos15(a.x))};
+  }
+}
+
 // multiply by the twiddle factor exp(DIR * 2 pi i m / 16), m a compile-time constant
 template <int DIR, int M, class C> __device__ __forceinline__ C tw16(C a) {
   using R = decltype(C::x);
@@ -157,7 +194,8 @@ template <int DIR, int M, class C> __device__ __forceinline__ C tw16(C a) {
   const R s1 = R(0.38268343236508977173);  // sin(pi/8)
   const R h = R(0.70710678118654752440);   // sqrt(1/2)
   // products with DIR = +-1 are written as sign changes (same bits)
-  if constexpr (m == 0) return a;
+  if constexpr (is_fx<C>::value) return fx_root<DIR, 3 * (m % 4)>(fx_quad<DIR, m / 4>(a));
+  else if constexpr (m == 0) return a;
   else if constexpr (m == 4) return crot<DIR>(a);
   else if constexpr (m == 8) return cmake<C>(-a.x, -a.y);
   else if constexpr (m == 12) return crot<-DIR>(a);
@@ -217,7 +255,9 @@ template <int DIR, int M, class C> __device__ __forceinline__ C tw32(C a) {
 template <int DIR, int M, class C> __device__ __forceinline__ C tw24(C a) {
   using R = decltype(C::x);
   constexpr int m = ((M % 24) + 24) % 24;
-  if constexpr (m == 0) {
+  if constexpr (is_fx<C>::value) {
+    return fx_root<DIR, 2 * (m % 6)>(fx_quad<DIR, m / 6>(a));
+  } else if constexpr (m == 0) {
     return a;
   } else if constexpr (m >= 6) {
     return crot<DIR>(tw24<DIR, m - 6>(a));  // exp(DIR i pi/2) = DIR * i
@@ -308,13 +348,18 @@ template <int DIR> struct Dft<2, DIR> {
 template <int DIR> struct Dft<3, DIR> {
   template <class C> __device__ __forceinline__ static void run(C* a) {
     using R = decltype(C::x);
-    const R half = R(0.5);
-    const R s3 = R(0.86602540378443864676);  // sqrt(3)/2
     const C t1 = cadd(a[1], a[2]);
     const C t2 = csub(a[1], a[2]);
-    const C m = cmake<C>(a[0].x - half * t1.x, a[0].y - half * t1.y);
-    // +/- i DIR sqrt(3)/2 (a1 - a2)
-    const C r = crot<DIR>(cscale(t2, s3));
+    C m, r;  // r = +/- i DIR sqrt(3)/2 (a1 - a2)
+    if constexpr (is_fx<C>::value) {
+      m = cmake<C>(a[0].x - (t1.x >> 1), a[0].y - (t1.y >> 1));
+      r = crot<DIR>(cmake<C>(fx_cos30(t2.x), fx_cos30(t2.y)));
+    } else {
+      const R half = R(0.5);
+      const R s3 = R(0.86602540378443864676);  // sqrt(3)/2
+      m = cmake<C>(a[0].x - half * t1.x, a[0].y - half * t1.y);
+      r = crot<DIR>(cscale(t2, s3));
+    }
     a[0] = cadd(a[0], t1);
     a[1] = cadd(m, r);
     a[2] = csub(m, r);
@@ -573,7 +618,19 @@ __device__ __forceinline__ void fft_stage(C (&v)[L][E], int j, const SM& sm, con
         } else {
           a[l][q][r] = sm.ld(l, j + q * T + r * (N / R));
         }
+        if constexpr (is_fx<C>::value && kFirst && FROM_SMEM)
+          a[l][q][r] = FxC{a[l][q][r].x << sm.pre, a[l][q][r].y << sm.pre};
       }
+  if constexpr (is_fx<C>::value && kLast && !kFirst) {
+    // room that the line's values left in front of the last stage
+    const int up = sm.up();
+#pragma unroll
+    for (int l = 0; l < L; ++l)
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[l][q][r] = FxC{a[l][q][r].x << up, a[l][q][r].y << up};
+  }
   if constexpr (!kFirst && SGPE_TW_FACTOR && Q > 1 && T * Q == NS) {
     // The Q butterflies of the thread sit at k = j + qT with NS = TQ, so
     // W_{NS R}^{(j + qT) r} = W_{NS R}^{j r} W_E^{q r}: R - 1 table values
@@ -598,6 +655,10 @@ __device__ __forceinline__ void fft_stage(C (&v)[L][E], int j, const SM& sm, con
       const int vt = j + q * T;
       using W = TwE<decltype(C::x)>;
       const W* twq = reinterpret_cast<const W*>(tw) + kOff + (vt % NS);
+      if constexpr (is_fx<C>::value) {  // the factor one, with the stage's scaling
+#pragma unroll
+        for (int l = 0; l < L; ++l) a[l][q][0] = fx_scale_down<fx_stage_bits(R, kLast)>(a[l][q][0]);
+      }
 #pragma unroll
       for (int r = 1; r < R; ++r) {
         const W w = __ldg(twq + (r - 1) * NS);

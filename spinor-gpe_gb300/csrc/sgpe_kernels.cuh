@@ -211,7 +211,22 @@ template <typename R> struct RowFields {
 
 enum RowMode { kRowStep = 0, kRowForward = 1, kRowInverse = 2 };
 
-template <typename R> struct RowArgs {
+// Fixed-point operands of a complex128 pass (sgpe_fx_kernels.cuh); empty for
+// the other precisions.  twf non-null selects the fixed-point kernels.
+template <typename R> struct RowFx {};
+template <> struct RowFx<double> {
+  const int4* twf;       // twiddles of the x transform as split factors
+  const int4* mf[4];     // RealOp::m times 2^(62 - me)
+  int me;
+};
+template <typename R> struct ColFx {};
+template <> struct ColFx<double> {
+  const int4* twf;
+  const int4* kb[2][2];  // [k1, k2][component] y-tables of the kinetic factors
+  int ke[2][2];          // times 2^(62 - ke); the x-tables are KinOp's own
+};
+
+template <typename R> struct RowArgs : RowFx<R> {
   const Cx<R>* in[2];
   Cx<R>* out[2];
   const Cx<R>* tw;        // per-stage twiddle table of the x transform
@@ -238,7 +253,7 @@ template <typename R> struct RowArgs {
   int* err;               // non-null: device error word (kErr* codes)
 };
 
-template <typename R> struct ColArgs {
+template <typename R> struct ColArgs : ColFx<R> {
   const Cx<R>* in[2];
   Cx<R>* out[2];
   const Cx<R>* tw;        // per-stage twiddle table of the y transform
@@ -982,6 +997,25 @@ row_kernel_grouped(const RowArgs<R>* __restrict__ args) {
 }
 
 // -------------------------------------------------------------- column pass
+// End of a block that wrote its partial sums (by thread 0): with ColArgs::fin
+// the last block to finish sums every block's partials (no block waits).
+template <typename R>
+__device__ __forceinline__ void col_finish(const ColArgs<R>& a, const BlockPos pos, int tid, int nthreads) {
+  if (a.fin == nullptr) return;
+  __shared__ bool s_last;
+  if (tid == 0) {
+    __threadfence();  // this block's partial is visible before its arrival
+    const unsigned ticket = atomicAdd(a.count, 1u);
+    s_last = (ticket == 2u * unsigned(pos.nx) - 1u);
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    final_sums(static_cast<const R*>(a.part), pos.nx, tid, nthreads, a.fin);
+    if (tid == 0) *a.count = 0u;
+  }
+}
+
 template <typename R, int N, int E, int COLS, bool TC = false, bool QUEUE = false>
 __device__ __forceinline__ void col_body(const ColArgs<R>& a, const BlockPos pos) {
   using C = Cx<R>;
@@ -1114,21 +1148,7 @@ __device__ __forceinline__ void col_body(const ColArgs<R>& a, const BlockPos pos
         dst[1] = bw;
       }
     }
-    if (a.fin != nullptr) {
-      // the last block to finish sums every block's partials (no block waits)
-      __shared__ bool s_last;
-      if (tid == 0) {
-        __threadfence();  // this block's partial is visible before its arrival
-        const unsigned ticket = atomicAdd(a.count, 1u);
-        s_last = (ticket == 2u * unsigned(pos.nx) - 1u);
-      }
-      __syncthreads();
-      if (s_last) {
-        __threadfence();
-        final_sums(static_cast<const R*>(a.part), pos.nx, tid, NT, a.fin);
-        if (tid == 0) *a.count = 0u;
-      }
-    }
+    col_finish(a, pos, tid, NT);
   }
 }
 

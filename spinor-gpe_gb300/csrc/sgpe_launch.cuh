@@ -4,13 +4,13 @@
 // 384 and 768, along either axis, instantiated for complex64 (float),
 // complex128 (double) and double-float (DF, kernel shape 0 only).
 #pragma once
-#include "sgpe_kernels.cuh"
+#include "sgpe_fx_kernels.cuh"
 
 namespace sgpe {
 
 // Points per thread E and the preferred column-tile width per precision.
 // complex64: E = 16, 8 columns (64-byte row segments per column tile);
-// complex128: E = 8, 4 columns (also 64-byte segments).  The complex64
+// complex128: E = 8, 2 columns.  The complex64
 // values can be overridden at compile time (-DSGPE_F32_...) for tuning sweeps.
 template <typename R> struct Tune;
 // ROW_MINB / COL_MINB: resident blocks per SM requested from the compiler
@@ -81,7 +81,9 @@ template <> struct Tune<float> {
 template <> struct Tune<double> {
   static constexpr int ROW_E = 8, ROW_THREADS = 256, ROW_MINB = SGPE_F64_ROW_MINB;
   static constexpr int ROW_E_LARGE = 8, ROW_MINB_LARGE = 2;
-  static constexpr int COL_E = 8, COLS = 4, COL_MINB = SGPE_F64_COL_MINB;
+  // 2 columns (32-byte row segments): the 1024^2 fixed-point column pass 70.7
+  // -> 63.8 us against 4, in four blocks per SM instead of two
+  static constexpr int COL_E = 8, COLS = 2, COL_MINB = SGPE_F64_COL_MINB;
   static constexpr int R3_E = 12, R3_ROW_MINB = 2, R3_COL_MINB = 1;
   static constexpr int R3_E_LARGE = 12, R3_COL_MINB_LARGE = 1;
   static constexpr int COL_MAX_THREADS = 1024, COL_MINB_LARGE = 1;
@@ -171,7 +173,7 @@ template <> struct ShapeTune<double> {
   static constexpr int row_minb(int, int) { return 0; }
   static constexpr int row_threads(int, int s) { return s == 2 ? 128 : Tune<double>::ROW_THREADS; }
   static constexpr int col_e(int, int) { return 4; }
-  static constexpr int cols(int, int s) { return s == 2 ? 2 : Tune<double>::COLS; }
+  static constexpr int cols(int, int s) { return s == 2 ? 2 : 4; }
 };
 // double-float: kernel shape 0 only
 template <> struct ShapeTune<DF> {
@@ -504,6 +506,76 @@ cudaError_t launch_col_grouped_s(const ColArgs<R>* args, int groups, int nx, int
   return dispatch_n(ny, ColGroupedLauncher<R, S>{args, groups, nx, s});
 }
 
+// Fixed-point complex128 passes: the tiles of the FP64 kernels' shapes at 64
+// registers (80 for the 12 points per thread of sides 3 * 2^k).  Measured at
+// 1024^2, step: 64 registers 400 us, 80 404 us, 128 422 us; at 768^2 80
+// registers 280 us, 64 435 us, 128 317 us.
+template <int E, int THREADS> constexpr int fx_minb() { return cmax(1, (E % 3 == 0 ? 768 : 1024) / THREADS); }
+
+template <int S> struct FxLauncher {
+  const RowArgs<double>* row;   // one of the two passes
+  const ColArgs<double>* col;
+  int groups;                   // 0: host arguments; else device arrays
+  int nx, ny;
+  cudaStream_t s;
+  template <int N> cudaError_t run() const { return row != nullptr ? run_row<N>() : run_col<N>(); }
+  template <int N> cudaError_t run_row() const {
+    using Cfg = RowCfg<double, N, S>;
+    if constexpr (!Cfg::VALID) {
+      return cudaErrorInvalidValue;
+    } else {
+      constexpr int MINB = fx_minb<Cfg::E, Cfg::THREADS>();
+      if (ny % Cfg::ROWS != 0) return cudaErrorInvalidValue;
+      auto k = row_kernel_fx<N, Cfg::E, Cfg::ROWS, MINB>;
+      auto kg = row_kernel_fx_grouped<N, Cfg::E, Cfg::ROWS, MINB>;
+      static unsigned long long done[2] = {0, 0};
+      cudaError_t e = groups ? smem_limit_once(kg, Cfg::SMEM, &done[1]) : smem_limit_once(k, Cfg::SMEM, &done[0]);
+      if (e != cudaSuccess) return e;
+      const dim3 grid(ny / Cfg::ROWS, groups ? groups : 1);
+      return groups ? launch_pdl(kg, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, row)
+                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *row);
+    }
+  }
+  template <int N> cudaError_t run_col() const {
+    using Cfg = ColCfg<double, N, S>;
+    if constexpr (!Cfg::VALID) {
+      return cudaErrorInvalidValue;
+    } else {
+      constexpr int MINB = fx_minb<Cfg::E, Cfg::THREADS>();
+      if (nx % Cfg::COLS != 0 || (nx / 2) % Cfg::COLS != 0) return cudaErrorInvalidValue;
+      auto k = col_kernel_fx<N, Cfg::E, Cfg::COLS, MINB>;
+      auto kg = col_kernel_fx_grouped<N, Cfg::E, Cfg::COLS, MINB>;
+      static unsigned long long done[2] = {0, 0};
+      cudaError_t e = groups ? smem_limit_once(kg, Cfg::SMEM, &done[1]) : smem_limit_once(k, Cfg::SMEM, &done[0]);
+      if (e != cudaSuccess) return e;
+      const dim3 grid(nx / Cfg::COLS, 2, groups ? groups : 1);
+      return groups ? launch_pdl(kg, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, col)
+                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *col);
+    }
+  }
+};
+template <int S>
+cudaError_t launch_row_fx_s(const RowArgs<double>* a, int groups, int nx, int ny, cudaStream_t s);
+template <int S>
+cudaError_t launch_col_fx_s(const ColArgs<double>* a, int groups, int nx, int ny, cudaStream_t s);
+#ifdef SGPE_FX_KERNELS
+template <int S>
+cudaError_t launch_row_fx_s(const RowArgs<double>* a, int groups, int nx, int ny, cudaStream_t s) {
+  return dispatch_n(nx, FxLauncher<S>{a, nullptr, groups, nx, ny, s});
+}
+template <int S>
+cudaError_t launch_col_fx_s(const ColArgs<double>* a, int groups, int nx, int ny, cudaStream_t s) {
+  return dispatch_n(ny, FxLauncher<S>{nullptr, a, groups, nx, ny, s});
+}
+#endif
+#define SGPE_EXTERN_FX(S)                                                                        \
+  extern template cudaError_t launch_row_fx_s<S>(const RowArgs<double>*, int, int, int, cudaStream_t); \
+  extern template cudaError_t launch_col_fx_s<S>(const ColArgs<double>*, int, int, int, cudaStream_t);
+SGPE_EXTERN_FX(0)
+SGPE_EXTERN_FX(1)
+SGPE_EXTERN_FX(2)
+#undef SGPE_EXTERN_FX
+
 #define SGPE_SHAPE_SWITCH(shape, CALL0, CALL1, CALL2) \
   switch (shape) {                                   \
     case 0: return CALL0;                            \
@@ -523,8 +595,20 @@ template <typename R, bool SEP> cudaError_t launch_row_ops(const RowArgs<R>& a, 
   }
 }
 
+inline cudaError_t launch_row_fx(const RowArgs<double>* a, int shape, int groups, int nx, int ny, cudaStream_t s) {
+  SGPE_SHAPE_SWITCH(shape, (launch_row_fx_s<0>(a, groups, nx, ny, s)), (launch_row_fx_s<1>(a, groups, nx, ny, s)),
+                    (launch_row_fx_s<2>(a, groups, nx, ny, s)))
+}
+inline cudaError_t launch_col_fx(const ColArgs<double>* a, int shape, int groups, int nx, int ny, cudaStream_t s) {
+  SGPE_SHAPE_SWITCH(shape, (launch_col_fx_s<0>(a, groups, nx, ny, s)), (launch_col_fx_s<1>(a, groups, nx, ny, s)),
+                    (launch_col_fx_s<2>(a, groups, nx, ny, s)))
+}
+
 template <typename R> cudaError_t launch_col(const ColArgs<R>& a, int ny, cudaStream_t s) {
   if (a.tc) return launch_col_tc(a, ny, s);
+  if constexpr (std::is_same<R, double>::value) {
+    if (a.twf != nullptr) return launch_col_fx(&a, a.shape, 0, a.nx, ny, s);
+  }
   if constexpr (is_df<R>::value) {
     return a.shape == 0 ? launch_col_s<R, 0>(a, ny, s) : cudaErrorInvalidValue;
   } else {
@@ -634,6 +718,9 @@ template <typename R> cudaError_t launch_row(const RowArgs<R>& a, int nx, int ny
   if (a.tc) {
     if (a.mode == kRowStep && !a.op.sep) return cudaErrorInvalidValue;  // not instantiated
     return launch_row_tc(a, nx, ny, s);
+  }
+  if constexpr (std::is_same<R, double>::value) {
+    if (a.twf != nullptr) return launch_row_fx(&a, a.shape, 0, nx, ny, s);
   }
   if (a.mode == kRowStep && !a.op.sep) return launch_row_ops<R, false>(a, nx, ny, s);
   return launch_row_ops<R, true>(a, nx, ny, s);
