@@ -168,6 +168,10 @@ struct sgpe_plan {
   int tc = 0;                // radix-16 stages on the tensor cores (split-BF16)
   int row_shape = 0;         // kernel shapes of the row (x) and column (y)
   int col_shape = 0;         // passes (sgpe_launch.cuh); twiddles follow them
+  // captured steps launch each pass after the previous one has ended
+  // (overlap_launches); eager steps always overlap the launches, whose host
+  // side would show otherwise
+  bool serial = false;
   uint32_t* tcb = nullptr;   // their B fragments (device)
   void* tw_x = nullptr;
   void* tw_y = nullptr;
@@ -829,6 +833,7 @@ template <typename R> bool col_step_args(sgpe_plan* p, int sub, bool want_u, sgp
   a.tc = p->tc;
   a.tcb = p->tcb;
   a.shape = p->col_shape;
+  a.serial = p->serial;
   a.tmap = (p->tmaps_valid && !p->tc) ? p->tmaps : nullptr;  // in place, no shifts
   a.err = p->derr;
   a.nx = p->nx;
@@ -873,6 +878,7 @@ template <typename R> sgpe::RowArgs<R> row_step_args(sgpe_plan* p, int sub, doub
   a.tc = p->tc;
   a.tcb = p->tcb;
   a.shape = p->row_shape;
+  a.serial = p->serial;
   a.err = p->derr;
   a.mode = sgpe::kRowStep;
   a.scale = R(1);
@@ -1102,6 +1108,7 @@ template <typename R> int fft2(sgpe_plan* p, const void* i0, const void* i1, voi
   c.tc = p->tc;
   c.tcb = p->tcb;
   c.shape = own ? p->col_shape : 0;
+  r.serial = c.serial = !sgpe::overlap_launches<R>(p->nx, p->ny, r.shape, c.shape);
   c.nx = p->nx;
   c.scale = R(1);
   if constexpr (std::is_same<R, double>::value) {
@@ -1266,7 +1273,9 @@ template <typename R> int capture_steps(sgpe_plan* p, int steps, cudaGraphExec_t
   cudaError_t e = cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "begin capture");
   int rc = SGPE_OK;
+  p->serial = !p->tc && !sgpe::overlap_launches<R>(p->nx, p->ny, p->row_shape, p->col_shape);
   for (int i = 0; i < steps && rc == SGPE_OK; ++i) rc = eager_step<R>(p, nullptr, p->cap_stream);
+  p->serial = false;
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(p->cap_stream, &graph);
   if (rc != SGPE_OK) {

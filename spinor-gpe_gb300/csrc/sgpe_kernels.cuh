@@ -250,6 +250,7 @@ template <typename R> struct RowArgs : RowFx<R> {
   int tc;                 // launch the tensor-core DFT16 kernels (host side)
   const uint32_t* tcb;    // their B fragments (kTcBfragWords, device)
   int shape;              // kernel shape of the launch (host side)
+  int serial;             // launch after the previous pass has ended (host side, overlap_launches)
   int* err;               // non-null: device error word (kErr* codes)
 };
 
@@ -275,6 +276,7 @@ template <typename R> struct ColArgs : ColFx<R> {
   int tc;                 // launch the tensor-core DFT16 kernels (host side)
   const uint32_t* tcb;    // their B fragments (kTcBfragWords, device)
   int shape;              // kernel shape of the launch (host side)
+  int serial;             // launch after the previous pass has ended (host side, overlap_launches)
   // non-null: two 2-D tensor maps (128 bytes each, device memory) of the
   // components, in == out, no shifts; box {2 COLS scalars, min(N, 256) rows}
   const void* tmap;

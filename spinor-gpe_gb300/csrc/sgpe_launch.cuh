@@ -257,9 +257,10 @@ template <class K> inline cudaError_t smem_limit_once(K kernel, size_t bytes, un
 }
 
 // Launch with programmatic stream serialisation (see SGPE_PDL), so the
-// kernel may be scheduled while its predecessor drains.
+// kernel may be scheduled while its predecessor drains; `serial`: without it.
 template <class K, class A>
-inline cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A& args) {
+inline cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A& args,
+                              bool serial = false) {
 #if SGPE_PDL
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -270,7 +271,7 @@ inline cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cuda
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = serial ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, args);
 #else
   kernel<<<grid, block, smem, s>>>(args);
@@ -301,7 +302,7 @@ template <typename R, bool SEP, int S> struct RowLauncher {
       static unsigned long long done = 0;
       cudaError_t e = smem_limit_once(k, Cfg::SMEM, &done);
       if (e != cudaSuccess) return e;
-      return launch_pdl(k, dim3(ny / Cfg::ROWS), dim3(Cfg::THREADS), Cfg::SMEM, s, *a);
+      return launch_pdl(k, dim3(ny / Cfg::ROWS), dim3(Cfg::THREADS), Cfg::SMEM, s, *a, a->serial != 0);
     }
   }
 };
@@ -321,7 +322,7 @@ template <typename R, int S> struct ColLauncher {
       static unsigned long long done = 0;
       cudaError_t e = smem_limit_once(k, Cfg::SMEM, &done);
       if (e != cudaSuccess) return e;
-      return launch_pdl(k, dim3(nx / Cfg::COLS, 2), dim3(Cfg::THREADS), Cfg::SMEM, s, *a);
+      return launch_pdl(k, dim3(nx / Cfg::COLS, 2), dim3(Cfg::THREADS), Cfg::SMEM, s, *a, a->serial != 0);
     }
   }
 };
@@ -533,7 +534,7 @@ template <int S> struct FxLauncher {
       if (e != cudaSuccess) return e;
       const dim3 grid(ny / Cfg::ROWS, groups ? groups : 1);
       return groups ? launch_pdl(kg, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, row)
-                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *row);
+                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *row, row->serial != 0);
     }
   }
   template <int N> cudaError_t run_col() const {
@@ -550,7 +551,7 @@ template <int S> struct FxLauncher {
       if (e != cudaSuccess) return e;
       const dim3 grid(nx / Cfg::COLS, 2, groups ? groups : 1);
       return groups ? launch_pdl(kg, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, col)
-                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *col);
+                    : launch_pdl(k, grid, dim3(Cfg::THREADS), Cfg::SMEM, s, *col, col->serial != 0);
     }
   }
 };
@@ -671,6 +672,28 @@ template <typename R> int col_tile_width(int ny, int shape = 0) {
   int re, ce, c;
   shape_geometry<R>(ny, shape, &re, &ce, &c);
   return c;
+}
+
+// Threads of both passes over an (ny, nx) grid.
+template <typename R> long long pass_threads(int nx, int ny, int rs, int cs) {
+  const long long points = 2ll * nx * ny;
+  return points / row_points_per_thread<R>(nx, rs) + points / col_points_per_thread<R>(ny, cs);
+}
+
+// Whether a plan's passes are launched while the previous one drains.  That
+// hides most of a launch (0.5 us of the 2.5 us of a 64^2 complex64 pass), but
+// the blocks are then placed wherever there is room first: a grid that fills
+// the GPU less than once piles up on the SMs that emptied first and runs as
+// long as the fullest of them.  Only passes short enough for the launch to
+// matter more are overlapped.  Measured in graphs (us a step, overlapped /
+// serial): complex64 128^2 15.9 / 19.0, 384^2 37.4 / 38.7 against 1024 x 256
+// 60.7 / 39.8, 1024 x 512 69.6 / 54.2, 512^2 38.3 / 36.1, 1024^2 88.5 / 85.0;
+// complex128 64^2 50.0 / 50.8 against 128 x 512 76.9 / 72.4, 512 x 256 176 /
+// 97, 512 x 768 269 / 204; double-float 64^2 98 / 79, 256^2 170 / 100, 512^2
+// 199 / 133, 2048^2 1793 / 1787.
+template <typename R> bool overlap_launches(int nx, int ny, int rs, int cs) {
+  if (is_df<R>::value) return false;
+  return pass_threads<R>(nx, ny, rs, cs) <= (sizeof(R) == 4 ? 49152 : 20480);
 }
 
 template <typename R> cudaError_t launch_scale(const ScaleArgs<R>& a, cudaStream_t s) {
