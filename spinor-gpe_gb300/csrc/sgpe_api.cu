@@ -157,11 +157,12 @@ struct sgpe_plan {
   double* fin = nullptr;     // their sums (3 doubles) and the pass's arrival
   unsigned* count = nullptr; // counter, behind the partials in `part`
   // the last column block forms the sums once and row blocks read them
-  // (double-float and complex128 plans, where every row block re-summing the
-  // partials cost ~10% of the double-float row pass and would be the
-  // fixed-point row pass's longest FP64 chain); complex64 row blocks sum the
-  // partials themselves while their other warps transform, which costs less
-  // than a serial tail on the column pass
+  // (double-float plans, where every row block re-summing the partials in
+  // double-float arithmetic cost ~10% of the row pass, and complex128 plans
+  // of 2048 columns and more: 2048^2 1,758 against 1,784 us a step); complex64
+  // and smaller complex128 row blocks sum the partials themselves while they
+  // wait, which costs less than a serial tail on the column pass (complex128
+  // 256^2 62 -> 55 us, 1024^2 426 -> 422 us a step)
   bool final_sums = false;
   int ntile = 0;             // column tiles of the current kernels
   int ntile_fp32 = 0;        // ... of the FP32 DFT kernels
@@ -803,10 +804,9 @@ void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops
 
 // Whether the row pass of sub-step `so` can run in fixed point: separable
 // operators with finite tables, an interaction factor that is a phase or
-// never above one (the point-wise results have no headroom to grow into),
-// and the column pass's final sums.
+// never above one (the point-wise results have no headroom to grow into).
 bool row_fx_ok(const sgpe_plan* p, const SubOps& so) {
-  if (p->bits != 128 || !p->final_sums || !fused_sep(so, p->coupling)) return false;
+  if (p->bits != 128 || !fused_sep(so, p->coupling)) return false;
   if (!(p->coupling ? so.sep.fx_c : so.sep.fx_d)) return false;
   if (so.zr == 0.0) return true;
   return so.zi == 0.0 && so.zr * p->g[0] <= 0.0 && so.zr * p->g[1] <= 0.0 && so.zr * p->g[2] <= 0.0;
@@ -817,6 +817,9 @@ template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowA
   const int4* m = static_cast<const int4*>(p->coupling ? so.sep.fm : so.sep.fdg);
   for (int k = 0; k < 4; ++k) a->mf[k] = m + (p->coupling ? k : k / 2) * p->nx;
   a->me = p->coupling ? so.sep.fme : so.sep.fdge;
+  const double z = (so.zi != 0.0 ? so.zi : so.zr) * a->norm_num;
+  for (int k = 0; k < 3; ++k) a->kz[k] = z * p->g[k];
+  a->sqrt_norm = std::sqrt(a->norm_num);
   a->twf = static_cast<const int4*>(p->twf_x);
 }
 
@@ -1423,7 +1426,7 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
   p->graphs_enabled = std::getenv("SGPE_DISABLE_GRAPHS") == nullptr;
   // SGPE_FINAL_SUMS=0/1 overrides the precision's choice (measurements)
   const char* fs = std::getenv("SGPE_FINAL_SUMS");
-  p->final_sums = fs != nullptr ? fs[0] == '1' : dtype_bits != 64;
+  p->final_sums = fs != nullptr ? fs[0] == '1' : dtype_bits == SGPE_DTYPE_DF || (dtype_bits == 128 && nx >= 2048);
   p->row_shape = default_shape(dtype_bits, 0, nx);
   p->col_shape = default_shape(dtype_bits, 1, ny);
   int cols = by_prec(dtype_bits, [&](auto t) { return sgpe::col_tile_width<decltype(t)>(ny, p->col_shape); });

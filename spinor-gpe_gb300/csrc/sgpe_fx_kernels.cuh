@@ -376,6 +376,35 @@ col_kernel_fx_grouped(const ColArgs<double>* __restrict__ args) {
 }
 
 // ----------------------------------------------------------------- row pass
+// Exact sums of non-negative FP64 values (the column pass's partials) over a
+// block: each value in 72 bits below the largest one's exponent, three limbs
+// of 24 bits whose sums over a warp (up to four values a thread) fit 32 bits.
+struct FxLimbs {
+  uint32_t l[3];
+};
+__device__ __forceinline__ void fx_limb_add(FxLimbs* s, double v, int be) {
+  const uint32_t hi = uint32_t(__double2hiint(v)), lo = uint32_t(__double2loint(v));
+  const uint64_t m = (uint64_t((hi << 11) | (lo >> 21) | 0x80000000u) << 32) | (lo << 11);
+  const int d = be - int(hi >> 20);        // below the largest exponent
+  const uint64_t t = fx_shr(m, d);         // the upper 64 bits
+  const uint64_t r = d == 0 ? 0 : d < 64 ? m << (64 - d) : fx_shr(m, d - 64);
+  s->l[0] += uint32_t(t >> 40);
+  s->l[1] += uint32_t(t >> 16) & 0xffffffu;
+  s->l[2] += (uint32_t(t & 0xffffu) << 8) | uint32_t(r >> 56);
+}
+// sum of the warps' limbs, times 2^q of one in the last of the 72 bits
+__device__ __forceinline__ double fx_limb_value(const FxLimbs* s, int stride, int warps, int be) {
+  uint64_t a = 0, b = 0, c = 0;
+  for (int w = 0; w < warps; ++w) {
+    a += s[w * stride].l[0];
+    b += s[w * stride].l[1];
+    c += s[w * stride].l[2];
+  }
+  // the largest exponent's values lie in [2^71, 2^72) units
+  const int q = be - 1023 - 71;
+  return fx_to_double(fx_t((a << 24) + b), q + 24) + fx_to_double(fx_t(c), q);
+}
+
 // What the point-wise operators of one row share.
 struct FxRow {
   int4 pb;           // pb(y) lambda
@@ -434,8 +463,11 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   FxC* sm = reinterpret_cast<FxC*>(smem_raw);
   __shared__ uint32_t s_mx[NT / 32];
   __shared__ uint32_t s_l1[NT / 32], s_l1f[2 * ROWS], s_mxf[2 * ROWS];
+  constexpr int NW = NT / 32;
+  __shared__ uint32_t s_wmax[NW];
+  __shared__ FxLimbs s_limb[NW][3];  // sums of w, u_0, u_1 per warp
   __shared__ FxRow s_row[ROWS];
-  __shared__ double s_lam2;
+  __shared__ double s_w;
 
   const int tid = threadIdx.x;
   const int rho = tid / (2 * T);
@@ -444,6 +476,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   const int y = pos.x * ROWS + rho;
   const long long row_off = (long long)y * N;
   const bool step = a.mode == kRowStep;
+  const bool want_u = a.pops != nullptr && pos.x == 0;
 
   FxC v[1][E];
   int q, q_other;   // exponents of this line and of the row's other component
@@ -455,6 +488,16 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
 #pragma unroll
     for (int m = 0; m < E; ++m) w[m] = in[row_off + j + m * T];
     allow_next_grid();
+    if (step && a.fin == nullptr) {
+      // the largest of the column pass's partial sums [comp][tile][u, w]
+      uint32_t wm = 0;
+      for (int i = tid; i < 2 * a.ntile; i += NT) {
+        wm = max(wm, uint32_t(__double2hiint(a.part[2 * i + 1])));
+        if (want_u) wm = max(wm, uint32_t(__double2hiint(a.part[2 * i])));
+      }
+      wm = __reduce_max_sync(0xffffffffu, wm);
+      if ((tid & 31) == 0) s_wmax[tid >> 5] = wm;
+    }
     if (tid < 2 * ROWS) s_l1f[tid] = s_mxf[tid] = 0;
     uint32_t mx = 0, other;
 #pragma unroll
@@ -507,13 +550,49 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   const FxC* tw = reinterpret_cast<const FxC*>(a.twf);
 
   if (step) {
+    int bw = 0;  // exponent of the largest partial
+    if (a.fin == nullptr) {
+      uint32_t wm = 0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) wm = max(wm, s_wmax[w]);
+      bw = max(int(wm >> 20), 2);
+      FxLimbs s[3] = {};
+      for (int i = tid; i < 2 * a.ntile; i += NT) {
+        fx_limb_add(&s[0], a.part[2 * i + 1], bw);
+        if (want_u) fx_limb_add(i < a.ntile ? &s[1] : &s[2], a.part[2 * i], bw);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k > 0 && !want_u) break;
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+          const uint32_t x = __reduce_add_sync(0xffffffffu, s[k].l[l]);
+          if ((tid & 31) == 0) s_limb[tid >> 5][k].l[l] = x;
+        }
+      }
+    }
     fft_lines<N, E, +1, 1, false, true>(v, j, smv, tw);
+    if constexpr (kWarp) __syncthreads();  // the limbs of every warp
     q += kTq - smv.shift;
     q_other += kTq - smv.shift_other;
     const int dq = 2 + a.me;  // the matrix tables are held as A 2^(62 - me)
     // the row's constants, by the first thread of each row
     if (comp == 0 && j == 0) {
-      const double lam2 = a.norm_num / a.fin[2], lam = sqrt(lam2);
+      double w;
+      if (a.fin != nullptr) w = a.fin[2];
+      else w = bw >= kFxNonFinite ? __hiloint2double(kNanHi, 0) : fx_limb_value(&s_limb[0][0], 3, NW, bw);
+      // y = sqrt(1/w) 2^h by one third-order step from the FP32 root of w 2^-2h
+      // in [1, 4) (FP64 operations are the longest chain of a small pass)
+      const int whi = __double2hiint(w);
+      const int h = ((whi >> 20) - 1023) >> 1;
+      const double wn = __hiloint2double(whi - (h << 21), __double2loint(w));
+      const int wnh = __double2hiint(wn);
+      const float y0 = rsqrtf(__int_as_float((((wnh >> 20) - 1023 + 127) << 23) | ((wnh & 0xfffff) << 3)));
+      const int yb = __float_as_int(y0);
+      const double ys = __hiloint2double((((yb >> 23) - 127 + 1023) << 20) | ((yb & 0x7fffff) >> 3), (yb & 7) << 29);
+      const double e = __fma_rn(-(wn * ys), ys, 1.0);
+      const double yw = __fma_rn(ys * e, __fma_rn(e, 0.375, 0.5), ys);
+      const double lam = a.sqrt_norm * yw, y2 = yw * yw;  // lambda 2^h, 2^2h / w
       FxRow& r = s_row[rho];
       const double2 mb = a.op.mb.p[y];
       const double px = mb.x * lam, py = mb.y * lam;
@@ -525,27 +604,37 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       r.pb = fx_factor(fx_from_words(xh, uint32_t(__double2loint(px)), be, 62),
                        fx_from_words(yh, uint32_t(__double2loint(py)), be, 62));
       const int qz[2] = {q, q_other};
-      const double z = (a.op.zi != 0.0 ? a.op.zi : a.op.zr) * lam2;
-      const double gs[2] = {a.g_uu, a.g_dd};
+      const double ko = a.kz[2] * y2;
+      const uint32_t oh = uint32_t(__double2hiint(ko));
+      uint32_t largest = oh & 0x7fffffffu;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         // phase_i = z (g_ik lambda^2 |z_k|^2) as hi64((|z_k|^2 << sh) m) 2^-64
-        const double kd = z * gs[k], ko = z * a.g_ud;
-        const uint32_t dh = uint32_t(__double2hiint(kd)), oh = uint32_t(__double2hiint(ko));
+        const double kd = a.kz[k] * y2;
+        const uint32_t dh = uint32_t(__double2hiint(kd));
+        largest = max(largest, dh & 0x7fffffffu);
         const int ek = int(max(dh & 0x7fffffffu, oh & 0x7fffffffu) >> 20) - 1022;
-        const int sh = max(0, ek + 2 * qz[k] + 129);
-        const int bk = 893 - 2 * qz[k] + sh;
-        r.sh[k] = min(sh, 62);
+        const int sh = max(0, ek + 2 * (qz[k] - h) + 129);
+        const int bk = 893 - 2 * (qz[k] - h) + sh;
         r.m[k][k] = fx_split(kd == 0.0 ? 0 : fx_from_words(dh, uint32_t(__double2loint(kd)), bk, 62));
         r.m[1 - k][k] = fx_split(ko == 0.0 ? 0 : fx_from_words(oh, uint32_t(__double2loint(ko)), bk, 62));
-        r.q[k] = qz[k] + dq + 64 + fx_line_q(be, 62);
-        if (sh > 62) r.sh[k] = 63;  // every nonzero density goes the FP64 way
+        r.sh[k] = sh > 62 ? 63 : sh;  // past 62 every nonzero density goes the FP64 way
+        r.q[k] = qz[k] + dq + 64 + fx_line_q(be, 62) - h;
       }
-      r.bad = be == kFxNonFinite || bad || !(lam2 < 1e300) || !(fabs(z) < 1e300);
+      r.bad = bad || be == kFxNonFinite || int(largest >> 20) == kFxNonFinite || whi < 0x100000 ||
+              (whi >> 20) == kFxNonFinite;
       if (tid == 0) {
-        s_lam2 = lam2;
-        if (a.pops != nullptr && pos.x == 0) {
-          const double u0 = a.fin[0], u1 = a.fin[1];
+        s_w = w;
+        if (want_u) {
+          double u0, u1;
+          if (a.fin != nullptr) {
+            u0 = a.fin[0];
+            u1 = a.fin[1];
+          } else {
+            const double nan = __hiloint2double(kNanHi, 0);
+            u0 = bw >= kFxNonFinite ? nan : fx_limb_value(&s_limb[0][1], 3, NW, bw);
+            u1 = bw >= kFxNonFinite ? nan : fx_limb_value(&s_limb[0][2], 3, NW, bw);
+          }
           a.pops[0] = a.atom_num * u0 / (u0 + u1);
           a.pops[1] = a.atom_num * u1 / (u0 + u1);
         }
@@ -613,7 +702,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
             z1 = fx_turn(x1, y1, z1, w1);
           }
         } else {
-          fx_point_far(&z0, &z1, q0, q1, dq, s_lam2, a, x);
+          fx_point_far(&z0, &z1, q0, q1, dq, a.norm_num / s_w, a, x);
         }
         z0 = fx_cmul<false>(z0, pb);
         z1 = fx_cmul<false>(z1, pb);

@@ -218,6 +218,8 @@ template <> struct RowFx<double> {
   const int4* twf;       // twiddles of the x transform as split factors
   const int4* mf[4];     // RealOp::m times 2^(62 - me)
   int me;
+  double kz[3];          // (zi or zr) norm_num (g_uu, g_dd, g_ud)
+  double sqrt_norm;      // sqrt(norm_num)
 };
 template <typename R> struct ColFx {};
 template <> struct ColFx<double> {
@@ -446,14 +448,40 @@ __device__ __forceinline__ void sum_partials(const DF* part, int ntile, int lane
   *w = from_df(c);
 }
 
-// lambda = sqrt(num / w) of the row pass, in the working precision.
+// The norm sum alone (the same additions in the same order as above).
+__device__ __forceinline__ FloatFloat sum_partials_w(const float* part, int ntile, int lane) {
+  FloatFloat sw;
+  for (int i0 = lane; i0 < 2 * ntile; i0 += 32 * kPartialBatch) {
+    float v[kPartialBatch];
+#pragma unroll
+    for (int k = 0; k < kPartialBatch; ++k) {
+      const int i = i0 + 32 * k;
+      v[k] = i < 2 * ntile ? part[2 * i + 1] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kPartialBatch; ++k) {
+      if (i0 + 32 * k >= 2 * ntile) break;
+      sw.add(v[k]);
+    }
+  }
+  sw.warp_reduce();
+  return sw;
+}
+
+// lambda = sqrt(num / w) of the row pass, in the working precision.  Warp 0
+// of every row block sums the partials while the block waits at the barrier
+// in front of the point-wise step, so the population sums are formed only
+// where they are written.
 __device__ __forceinline__ float row_lambda(const float* part, int ntile, int lane, float norm_num, double* u0,
                                             double* u1, bool want_u) {
-  FloatFloat a, b, c;
-  sum_partials(part, ntile, lane, &a, &b, &c);
+  FloatFloat c;
   if (want_u) {
+    FloatFloat a, b;
+    sum_partials(part, ntile, lane, &a, &b, &c);
     *u0 = a.value();
     *u1 = b.value();
+  } else {
+    c = sum_partials_w(part, ntile, lane);
   }
   return sqrtf(norm_num / (c.hi + c.lo));
 }
