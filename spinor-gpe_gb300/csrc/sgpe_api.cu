@@ -823,6 +823,13 @@ template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowA
   a->twf = static_cast<const int4*>(p->twf_x);
 }
 
+// The sums that the row pass of sub-step `sub` reads, or null when it adds up
+// the column pass's partials itself: the FP64 rows of a complex128 plan read
+// them (an FP64 sum of the partials in every row block costs them more).
+double* step_fin(const sgpe_plan* p, int sub) {
+  return p->final_sums || (p->bits == 128 && !row_fx_ok(p, p->sub[sub])) ? p->fin : nullptr;
+}
+
 // Column pass over the state (in place) ending a sub-step and starting `sub`.
 // want_u: the populations of the state entering the pass are needed, so the
 // two kinetic half steps are applied separately (sum after the first).
@@ -863,7 +870,7 @@ template <typename R> bool col_step_args(sgpe_plan* p, int sub, bool want_u, sgp
   }
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
-  a.fin = p->final_sums ? p->fin : nullptr;
+  a.fin = step_fin(p, sub);
   a.count = p->count;
   return true;
 }
@@ -891,7 +898,7 @@ template <typename R> sgpe::RowArgs<R> row_step_args(sgpe_plan* p, int sub, doub
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
   a.ntile = p->ntile;
-  a.fin = p->final_sums ? p->fin : nullptr;
+  a.fin = step_fin(p, sub);
   a.norm_num = p->atom_num / (double(p->nx) * double(p->ny) * p->dv_r);
   a.g_uu = R(p->g[0]);
   a.g_dd = R(p->g[1]);
