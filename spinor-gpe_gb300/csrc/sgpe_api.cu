@@ -1578,6 +1578,22 @@ int sgpe_set_dft_mode(sgpe_plan* p, int mode) {
       return cuda_fail(e, "tensor-core DFT tables");
     }
   }
+  if (mode != p->tc) {
+    // the column transforms of the two modes can differ in points per thread
+    const int e_tc = sgpe::tc_col_points_per_thread(p->ny), e_fp = sgpe::col_points_per_thread<float>(p->ny, p->col_shape);
+    if (e_tc != e_fp) {
+      DeviceGuard g(p->device);
+      cudaError_t e = cudaSuccess;
+      void* t = upload_twiddles<float>(p->ny, mode ? e_tc : e_fp, &e);
+      if (e != cudaSuccess) {
+        if (t) cudaFree(t);
+        return fail(SGPE_ERR_OOM, std::string("twiddle tables: ") + cudaGetErrorString(e));
+      }
+      drop_graphs(p);
+      cudaFree(p->tw_y);  // waits for launches still reading it
+      p->tw_y = t;
+    }
+  }
   p->tc = mode;
   p->ntile = mode ? p->nx / sgpe::tc_col_tile_width(p->ny) : p->ntile_fp32;
   drop_graphs(p);

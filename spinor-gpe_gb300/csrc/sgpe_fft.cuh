@@ -231,23 +231,35 @@ template <int DIR, class C> __device__ __forceinline__ C tw16r(C a, int m) {
   }
 }
 
-// multiply by exp(DIR * 2 pi i m / 32), m a compile-time constant
+// multiply by exp(DIR * 2 pi i m / 32), m a compile-time constant.
+//
+// In FP32 the rounded cosine and sine of a constant root scale every value
+// they meet alike, in the forward and in the inverse transform of every step:
+// with the nearest pairs in both, their product is off one by up to 5.8e-8
+// (pi/8 and pi/16), which adds up step by step.  The two directions therefore
+// take neighbouring pairs whose product is within 1.1e-8 of one, each still
+// within 4e-8 of its root.  (20 transform pairs of 1024 points in FP32: 9e-7
+// against 1.4e-6 with the nearest pairs, and 1.0e-6 for radices 16, 16, 4.)
 template <int DIR, int M, class C> __device__ __forceinline__ C tw32(C a) {
   using R = decltype(C::x);
-  constexpr int m = M & 31;
-  if constexpr (m % 2 == 0) {
-    return tw16<DIR, m / 2>(a);
-  } else if constexpr (m > 8) {
+  constexpr int m = M & 31, q = m % 8;
+  if constexpr (m >= 8) {
     return crot<DIR>(tw32<DIR, m - 8>(a));  // exp(DIR i pi/2) = DIR * i
+  } else if constexpr (q == 0) {
+    return a;
+  } else if constexpr (q == 4) {
+    return tw16<DIR, 2>(a);
   } else {
-    const R c1 = R(0.98078528040323044913);  // cos(pi/16)
-    const R s1 = R(0.19509032201612826785);  // sin(pi/16)
-    const R c3 = R(0.83146961230254523708);  // cos(3 pi/16)
-    const R s3 = R(0.55557023301960222474);  // sin(3 pi/16)
-    if constexpr (m == 1) return cmul(a, cmake<C>(c1, sgn<DIR>(s1)));
-    else if constexpr (m == 3) return cmul(a, cmake<C>(c3, sgn<DIR>(s3)));
-    else if constexpr (m == 5) return cmul(a, cmake<C>(s3, sgn<DIR>(c3)));  // cos(5pi/16) = sin(3pi/16)
-    else return cmul(a, cmake<C>(s1, sgn<DIR>(c1)));                        // m == 7
+    // cosine and sine of pi m / 16; in FP32 the double literals name the
+    // neighbours exactly
+    constexpr bool f32 = sizeof(R) == 4;
+    constexpr double c1 = f32 && DIR > 0 ? 0.9807853102684021 : 0.98078528040323044913;
+    constexpr double s1 = f32 && DIR < 0 ? 0.19509030878543854 : 0.19509032201612826785;
+    constexpr double c2 = f32 && DIR > 0 ? 0.92387956380844116 : 0.92387953251128675613;
+    constexpr double s2 = f32 && DIR > 0 ? 0.38268345594406128 : 0.38268343236508977173;
+    constexpr double c3 = 0.83146961230254523708, s3 = 0.55557023301960222474;
+    constexpr double co[8] = {1.0, c1, c2, c3, 0.0, s3, s2, s1}, si[8] = {0.0, s1, s2, s3, 0.0, c3, c2, c1};
+    return cmul(a, cmake<C>(R(co[q]), sgn<DIR>(R(si[q]))));
   }
 }
 
@@ -424,35 +436,42 @@ template <int DIR> struct Dft<16, DIR> {
 
 template <int DIR> struct Dft<32, DIR> {
   template <class C> __device__ __forceinline__ static void run(C* a) {
-    // decimation in time: DFT16 of the even and of the odd points, then
-    // a[k] = e[k] + W32^k o[k], a[k + 16] = e[k] - W32^k o[k]
-    C e[16], o[16];
+    // n = n2 + 8 n1, k = k1 + 4 k2: inner DFT4 over n1, twiddle W32^{n2 k1},
+    // outer DFT8 over n2 (fewer products than two DFT16)
+    C b[4][8];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      e[k] = a[2 * k];
-      o[k] = a[2 * k + 1];
+    for (int n2 = 0; n2 < 8; ++n2) {
+      C t[4] = {a[n2], a[n2 + 8], a[n2 + 16], a[n2 + 24]};
+      Dft<4, DIR>::run(t);
+#pragma unroll
+      for (int k1 = 0; k1 < 4; ++k1) b[k1][n2] = t[k1];
     }
-    Dft<16, DIR>::run(e);
-    Dft<16, DIR>::run(o);
-    o[1] = tw32<DIR, 1>(o[1]);
-    o[2] = tw32<DIR, 2>(o[2]);
-    o[3] = tw32<DIR, 3>(o[3]);
-    o[4] = tw32<DIR, 4>(o[4]);
-    o[5] = tw32<DIR, 5>(o[5]);
-    o[6] = tw32<DIR, 6>(o[6]);
-    o[7] = tw32<DIR, 7>(o[7]);
-    o[8] = tw32<DIR, 8>(o[8]);
-    o[9] = tw32<DIR, 9>(o[9]);
-    o[10] = tw32<DIR, 10>(o[10]);
-    o[11] = tw32<DIR, 11>(o[11]);
-    o[12] = tw32<DIR, 12>(o[12]);
-    o[13] = tw32<DIR, 13>(o[13]);
-    o[14] = tw32<DIR, 14>(o[14]);
-    o[15] = tw32<DIR, 15>(o[15]);
+    b[1][1] = tw32<DIR, 1>(b[1][1]);
+    b[1][2] = tw32<DIR, 2>(b[1][2]);
+    b[1][3] = tw32<DIR, 3>(b[1][3]);
+    b[1][4] = tw32<DIR, 4>(b[1][4]);
+    b[1][5] = tw32<DIR, 5>(b[1][5]);
+    b[1][6] = tw32<DIR, 6>(b[1][6]);
+    b[1][7] = tw32<DIR, 7>(b[1][7]);
+    b[2][1] = tw32<DIR, 2>(b[2][1]);
+    b[2][2] = tw32<DIR, 4>(b[2][2]);
+    b[2][3] = tw32<DIR, 6>(b[2][3]);
+    b[2][4] = tw32<DIR, 8>(b[2][4]);
+    b[2][5] = tw32<DIR, 10>(b[2][5]);
+    b[2][6] = tw32<DIR, 12>(b[2][6]);
+    b[2][7] = tw32<DIR, 14>(b[2][7]);
+    b[3][1] = tw32<DIR, 3>(b[3][1]);
+    b[3][2] = tw32<DIR, 6>(b[3][2]);
+    b[3][3] = tw32<DIR, 9>(b[3][3]);
+    b[3][4] = tw32<DIR, 12>(b[3][4]);
+    b[3][5] = tw32<DIR, 15>(b[3][5]);
+    b[3][6] = tw32<DIR, 18>(b[3][6]);
+    b[3][7] = tw32<DIR, 21>(b[3][7]);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      a[k] = cadd(e[k], o[k]);
-      a[k + 16] = csub(e[k], o[k]);
+    for (int k1 = 0; k1 < 4; ++k1) {
+      Dft<8, DIR>::run(b[k1]);
+#pragma unroll
+      for (int k2 = 0; k2 < 8; ++k2) a[k1 + 4 * k2] = b[k1][k2];
     }
   }
 };

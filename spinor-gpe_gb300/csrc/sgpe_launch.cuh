@@ -135,6 +135,17 @@ template <typename R> constexpr int pick_e(int n, int e_pow2) {
   return (n % 3 == 0) ? (n >= 768 ? Tune<R>::R3_E_LARGE : Tune<R>::R3_E) : cmin(n, e_pow2);
 }
 
+// ... of the column transform in kernel shape 0.  complex64 columns of 1024
+// take 32: two radix-32 stages with one exchange instead of three stages with
+// two, at 128 registers (two 256-thread blocks of 8 columns per SM; at 80
+// registers it spills).  The column pass, which waits for shared memory as
+// much as it issues, took 14.2 -> 12.4 us at 1024^2 (step 83.9 -> 78.5 us).  At
+// 2048 and 4096 either plan has three stages, and rows of 1024, with the
+// point-wise step between their transforms, are slower with 32.
+template <typename R> constexpr int pick_col_e(int n) {
+  return sizeof(R) == 4 && n == 1024 ? 32 : pick_e<R>(n, Tune<R>::COL_E);
+}
+
 // Kernel shapes.  A pass over lines of one length can run in several
 // shapes: launch configurations that differ in points per thread E (and so in
 // the radix plan and the twiddle tables) and in lines per block.  Shape 0 is
@@ -207,7 +218,7 @@ template <typename R, int N, int S = 0> struct RowCfg {
 
 template <typename R, int N, int S = 0> struct ColCfg {
   static constexpr bool VALID = S < col_shape_count<R>(N);
-  static constexpr int E = S == 0 ? pick_e<R>(N, Tune<R>::COL_E) : cmin(N, ShapeTune<R>::col_e(N, S));
+  static constexpr int E = S == 0 ? pick_col_e<R>(N) : cmin(N, ShapeTune<R>::col_e(N, S));
   static constexpr int T = N / E;
   static constexpr int COLS =
       cmax(cmin(S == 0 ? Tune<R>::COLS : ShapeTune<R>::cols(N, S), Tune<R>::COL_MAX_THREADS / T), 32 / T);
@@ -441,6 +452,8 @@ struct ColTcColsQuery {
     return cudaSuccess;
   }
 };
+// Points per thread of the tensor-core column transform.
+inline int tc_col_points_per_thread(int ny) { return pick_e<float>(ny, Tune<float>::COL_E); }
 // Column-tile width of the tensor-core column kernels (0 if unsupported).
 inline int tc_col_tile_width(int ny) {
   int c = 0;
