@@ -88,33 +88,60 @@ __device__ __forceinline__ uint32_t fx_hi_max(uint32_t m, int4 w) {
   const uint32_t a = uint32_t(w.y) & 0x7fffffffu, b = uint32_t(w.w) & 0x7fffffffu;
   return max(m, max(a, b));
 }
-__device__ __forceinline__ FxC fx_load(int4 w, int be, int p) {
-  return FxC{fx_from_words(uint32_t(w.y), uint32_t(w.x), be, p), fx_from_words(uint32_t(w.w), uint32_t(w.z), be, p)};
+// FP64 <-> integer through the conversion instructions: at 48 cycles of the
+// otherwise idle FP64 pipe they leave the integer pipes, which bound these
+// kernels, 7 instructions a value instead of 39 (sgpe_fx.cuh's word forms).
+// The power of two goes into the exponent field.  Where the pipe would be
+// waited for, the word forms stay: with 12 points per thread (sides 3 * 2^k:
+// a 768^2 transform pair 98 against 108 us), in the small shapes of 4,
+// with a few warps per SM, and on lines of 4096, whose one block per SM
+// converts all at once (us a step, instructions / words: 1024^2 411 / 422;
+// 2048^2 1,754 / 1,778; 256^2 56.4 / 53.3, 4096^2 8,300 / 7,858).
+__host__ __device__ constexpr bool fx_convert(int n, int e) { return e == 8 && n <= 2048; }
+__device__ __forceinline__ fx_t fx_load_part(uint32_t hi, uint32_t lo, int q) {
+  const int e = q << 20;
+  // below the normal range after the scaling: reads as zero (2^-62 of the line)
+  const bool tiny = int(hi & 0x7fffffffu) - e < 0x100000;
+  return __double2ll_rn(__hiloint2double(tiny ? 0 : int(hi) - e, int(lo)));
+}
+// a value of a line of biased exponent be at |part| < 2^p
+template <bool CONVERT> __device__ __forceinline__ FxC fx_load(int4 w, int be, int p) {
+  if constexpr (CONVERT) {
+    const int q = fx_line_q(be, p);
+    return FxC{fx_load_part(uint32_t(w.y), uint32_t(w.x), q), fx_load_part(uint32_t(w.w), uint32_t(w.z), q)};
+  } else {
+    return FxC{fx_from_words(uint32_t(w.y), uint32_t(w.x), be, p), fx_from_words(uint32_t(w.w), uint32_t(w.z), be, p)};
+  }
 }
 // v 2^q for any q (overflow to infinity, underflow to zero)
-static __device__ __noinline__ double fx_to_double_far(fx_t v, int q) { return ldexp(ldexp(double(v), q / 2), q - q / 2); }
-__device__ __forceinline__ double fx_to_double(fx_t v, int q) {
-  if (!fx_q_safe(q)) return fx_to_double_far(v, q);
-  uint32_t hi, lo;
-  fx_to_words(v, q, &hi, &lo);
-  return __hiloint2double(int(hi), int(lo));
+static __device__ __noinline__ double fx_to_double_far(fx_t v, int q) {
+  return ldexp(ldexp(double(v), q / 2), q - q / 2);
 }
-__device__ __forceinline__ int4 fx_words(FxC v, int q, bool safe) {
-  uint32_t xh, xl, yh, yl;
-  if (safe) {
+// ... for q in the range of fx_q_safe
+__device__ __forceinline__ double fx_to_double_near(fx_t v, int q) {
+  const double d = __ll2double_rn(v);
+  const int hi = __double2hiint(d);
+  return __hiloint2double(v == 0 ? 0 : hi + (q << 20), __double2loint(d));
+}
+__device__ __forceinline__ double fx_to_double(fx_t v, int q) {
+  return fx_q_safe(q) ? fx_to_double_near(v, q) : fx_to_double_far(v, q);
+}
+// What a line's element is written as: v 2^q, or NaN in a bad line.
+enum FxOut { kFxNear = 0, kFxFar = 1, kFxBad = 2 };
+__device__ __forceinline__ FxOut fx_out(bool bad, int q) { return bad ? kFxBad : fx_q_safe(q) ? kFxNear : kFxFar; }
+template <FxOut OUT, bool CONVERT> __device__ __forceinline__ int4 fx_words(FxC v, int q) {
+  if constexpr (OUT == kFxBad) return make_int4(0, 0x7ff80000, 0, 0x7ff80000);
+  if constexpr (OUT == kFxNear && !CONVERT) {
+    uint32_t xh, xl, yh, yl;
     fx_to_words(v.x, q, &xh, &xl);
     fx_to_words(v.y, q, &yh, &yl);
-  } else {
-    const double x = fx_to_double_far(v.x, q), y = fx_to_double_far(v.y, q);
-    xh = uint32_t(__double2hiint(x));
-    xl = uint32_t(__double2loint(x));
-    yh = uint32_t(__double2hiint(y));
-    yl = uint32_t(__double2loint(y));
+    return make_int4(int(xl), int(xh), int(yl), int(yh));
   }
-  return make_int4(int(xl), int(xh), int(yl), int(yh));
+  const double x = OUT == kFxNear ? fx_to_double_near(v.x, q) : fx_to_double_far(v.x, q);
+  const double y = OUT == kFxNear ? fx_to_double_near(v.y, q) : fx_to_double_far(v.y, q);
+  return make_int4(__double2loint(x), __double2hiint(x), __double2loint(y), __double2hiint(y));
 }
 constexpr int kNanHi = 0x7ff80000;
-__device__ __forceinline__ int4 fx_nan_words() { return make_int4(0, kNanHi, 0, kNanHi); }
 
 // A real factor as a mantissa |m| < 2^62 and its exponent.
 struct FxScale {
@@ -178,7 +205,7 @@ __device__ __forceinline__ int fx_kinetic(FxC (&v)[E], const double2* __restrict
                                           int eb, int x, int j) {
   const int4 w = __ldg(reinterpret_cast<const int4*>(ka) + x);
   const int be = fx_line_exp(fx_hi_max(0, w));
-  const FxC a = fx_load(w, be, 61);
+  const FxC a = fx_load<false>(w, be, 61);
   const FxSplit ax = fx_split(a.x), ay = fx_split(a.y);
 #pragma unroll
   for (int m = 0; m < E; ++m) {
@@ -265,7 +292,7 @@ __device__ __forceinline__ void col_body_fx(const ColArgs<double>& a, const Bloc
     const int p = (!a.fwd && a.nk > 0) ? 63 - kBits : 62 - kBits;
     q = fx_line_q(be, p);
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[0][m] = fx_load(w[m], be, p);
+    for (int m = 0; m < E; ++m) v[0][m] = fx_load<fx_convert(N, E)>(w[m], be, p);
   }
   const FxC* tw = reinterpret_cast<const FxC*>(a.twf);
   using Line = FxLine<N, E, false, false>;
@@ -323,15 +350,21 @@ __device__ __forceinline__ void col_body_fx(const ColArgs<double>& a, const Bloc
     qo += 64 + s.e;
     bad = bad || !s.finite;
   }
-  const bool safe = fx_q_safe(qo);
   {
     const long long step = (long long)T * nx, swap = a.out_shift ? E / 2 * step : 0;
-    int4* p = out + (long long)j * nx + xout + swap;
+    int4* const first = out + (long long)j * nx + xout + swap;
+    auto write = [&](auto form) {
+      int4* p = first;
 #pragma unroll
-    for (int m = 0; m < E; ++m, p += step) {
-      if (m == E / 2) p -= 2 * swap;
-      *p = bad ? fx_nan_words() : fx_words(v[0][m], qo, safe);
-    }
+      for (int m = 0; m < E; ++m, p += step) {
+        if (m == E / 2) p -= 2 * swap;
+        *p = fx_words<decltype(form)::value, fx_convert(N, E)>(v[0][m], qo);
+      }
+    };
+    const FxOut form = fx_out(bad, qo);
+    if (form == kFxNear) write(std::integral_constant<FxOut, kFxNear>{});
+    else if (form == kFxBad) write(std::integral_constant<FxOut, kFxBad>{});
+    else write(std::integral_constant<FxOut, kFxFar>{});
   }
   if (a.part != nullptr) {
     sw = fx_column_sum<COLS>(sw);
@@ -408,12 +441,24 @@ __device__ __forceinline__ double fx_limb_value(const FxLimbs* s, int stride, in
 // What the point-wise operators of one row share.
 struct FxRow {
   int4 pb;           // pb(y) lambda
-  FxSplit m[2][2];   // phase of component i per |z_j|^2
+  FxSplit m[2][2];   // phase of component i per |z_j|^2 (times 2^-twice)
   int sh[2];         // |z_j|^2 is shifted left by this before the product
+  int twice;         // the phases come out times 2^-twice
   int q[2];          // exponent of the components' lines in front of F_x
   bool bad;
 };
 
+// e^{i 2^twice x} - 1 as a split factor, x = X 2^-64, the phase at most 1/2
+__device__ __forceinline__ int4 fx_phase(fx_t X, int twice) {
+  fx_t sn, cm;
+  fx_sincos(X, &sn, &cm);
+  for (int k = 0; k < twice; ++k) {  // sin 2x = 2 (sin x + sin x (cos x - 1)), cos 2x - 1 = -2 sin^2 x
+    const FxSplit s = fx_split(sn);
+    sn = fx_mul(s, fx_split(cm), sn) << 1;
+    cm = -(fx_mul(s, s) << 1);
+  }
+  return fx_factor(cm, sn);
+}
 // |z|^2 in units of 2^63
 __device__ __forceinline__ fx_t fx_abs2(FxSplit x, FxSplit y) {
   const fx_t hl = fx_mad(x.h, x.l, fx_mad(y.h, y.l, 0));
@@ -428,27 +473,26 @@ __device__ __forceinline__ FxC fx_grow(FxSplit x, FxSplit y, FxC z, FxSplit w) {
 
 // The interaction, matrix, interaction sequence in FP64, for a point whose
 // phases are too large for the series of fx_sincos / fx_expm1.  z comes with
-// exponents q and goes with exponents q + dq.
-static __device__ __noinline__ void fx_point_far(FxC* z0, FxC* z1, int q0, int q1, int dq, double lam2,
-                                          const RowArgs<double>& a, int x) {
-  double2 p0 = make_double2(fx_to_double_far(z0->x, q0), fx_to_double_far(z0->y, q0));
-  double2 p1 = make_double2(fx_to_double_far(z1->x, q1), fx_to_double_far(z1->y, q1));
+// exponents q and goes with exponents q + dq; m: the matrix, m01 and m10
+// unread (zero) without coupling.  (By value: an address would keep the points
+// of the common path in local memory.)
+struct FxPair {
+  FxC z0, z1;
+};
+static __device__ __noinline__ FxPair fx_point_far(FxPair z, int q0, int q1, int dq, double lam2, double zr, double zi,
+                                                   double g_uu, double g_dd, double g_ud, double2 m00, double2 m01,
+                                                   double2 m10, double2 m11) {
+  double2 p0 = make_double2(fx_to_double_far(z.z0.x, q0), fx_to_double_far(z.z0.y, q0));
+  double2 p1 = make_double2(fx_to_double_far(z.z1.x, q1), fx_to_double_far(z.z1.y, q1));
   const double n0 = lam2 * cabs2(p0), n1 = lam2 * cabs2(p1);
-  const double2 i0 = cexp_z<double>(a.op.zr, a.op.zi, a.g_uu * n0 + a.g_ud * n1);
-  const double2 i1 = cexp_z<double>(a.op.zr, a.op.zi, a.g_dd * n1 + a.g_ud * n0);
+  const double2 i0 = cexp_z<double>(zr, zi, g_uu * n0 + g_ud * n1);
+  const double2 i1 = cexp_z<double>(zr, zi, g_dd * n1 + g_ud * n0);
   p0 = cmul(p0, i0);
   p1 = cmul(p1, i1);
-  double2 r0 = cmul(a.op.m[0].p[x], p0), r1 = cmul(a.op.m[3].p[x], p1);
-  if (!a.op.diag) {
-    r0 = cadd(r0, cmul(a.op.m[1].p[x], p1));
-    r1 = cadd(r1, cmul(a.op.m[2].p[x], p0));
-  }
-  r0 = cmul(r0, i0);
-  r1 = cmul(r1, i1);
-  z0->x = __double2ll_rn(ldexp(r0.x, -(q0 + dq)));
-  z0->y = __double2ll_rn(ldexp(r0.y, -(q0 + dq)));
-  z1->x = __double2ll_rn(ldexp(r1.x, -(q1 + dq)));
-  z1->y = __double2ll_rn(ldexp(r1.y, -(q1 + dq)));
+  const double2 r0 = cmul(cadd(cmul(m00, p0), cmul(m01, p1)), i0);
+  const double2 r1 = cmul(cadd(cmul(m11, p1), cmul(m10, p0)), i1);
+  return FxPair{FxC{__double2ll_rn(ldexp(r0.x, -(q0 + dq))), __double2ll_rn(ldexp(r0.y, -(q0 + dq)))},
+                FxC{__double2ll_rn(ldexp(r1.x, -(q1 + dq))), __double2ll_rn(ldexp(r1.y, -(q1 + dq)))}};
 }
 
 template <int N, int E, int ROWS>
@@ -528,7 +572,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
     q = fx_line_q(be, 62 - kBits);
     q_other = fx_line_q(be_other, 62 - kBits);
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[0][m] = fx_load(w[m], be, 62 - kBits);
+    for (int m = 0; m < E; ++m) v[0][m] = fx_load<fx_convert(N, E)>(w[m], be, 62 - kBits);
   }
   constexpr bool kWarp = (32 % T == 0);
   constexpr int WL = T < 32 ? 0 : T / 32;  // entries of s_l1 that make up a line
@@ -556,19 +600,19 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
 #pragma unroll
       for (int w = 0; w < NW; ++w) wm = max(wm, s_wmax[w]);
       bw = max(int(wm >> 20), 2);
-      FxLimbs s[3] = {};
-      for (int i = tid; i < 2 * a.ntile; i += NT) {
-        fx_limb_add(&s[0], a.part[2 * i + 1], bw);
-        if (want_u) fx_limb_add(i < a.ntile ? &s[1] : &s[2], a.part[2 * i], bw);
-      }
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (k > 0 && !want_u) break;
+      auto warp_limbs = [&](int k, int i0, int i1, int part) {
+        FxLimbs s{};
+        for (int i = i0 + tid; i < i1; i += NT) fx_limb_add(&s, a.part[2 * i + part], bw);
 #pragma unroll
         for (int l = 0; l < 3; ++l) {
-          const uint32_t x = __reduce_add_sync(0xffffffffu, s[k].l[l]);
+          const uint32_t x = __reduce_add_sync(0xffffffffu, s.l[l]);
           if ((tid & 31) == 0) s_limb[tid >> 5][k].l[l] = x;
         }
+      };
+      warp_limbs(0, 0, 2 * a.ntile, 1);
+      if (want_u) {
+        warp_limbs(1, 0, a.ntile, 0);
+        warp_limbs(2, a.ntile, 2 * a.ntile, 0);
       }
     }
     fft_lines<N, E, +1, 1, false, true>(v, j, smv, tw);
@@ -606,17 +650,26 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       const int qz[2] = {q, q_other};
       const double ko = a.kz[2] * y2;
       const uint32_t oh = uint32_t(__double2hiint(ko));
+      const uint32_t dh[2] = {uint32_t(__double2hiint(a.kz[0] * y2)), uint32_t(__double2hiint(a.kz[1] * y2))};
+      const uint32_t dl[2] = {uint32_t(__double2loint(a.kz[0] * y2)), uint32_t(__double2loint(a.kz[1] * y2))};
       uint32_t largest = oh & 0x7fffffffu;
+      int raw[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        largest = max(largest, dh[k] & 0x7fffffffu);
+        raw[k] = int(max(dh[k] & 0x7fffffffu, oh & 0x7fffffffu) >> 20) - 1022 + 2 * (qz[k] - h) + 129;
+      }
+      // |z|^2 is below 2^58 units: with shifts up to 4 no phase can leave the
+      // series' range, and up to two doublings keep the shifts there for
+      // phases up to 1/2
+      const int twice = min(2, max(0, max(raw[0], raw[1]) - 4));
+      r.twice = twice;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         // phase_i = z (g_ik lambda^2 |z_k|^2) as hi64((|z_k|^2 << sh) m) 2^-64
-        const double kd = a.kz[k] * y2;
-        const uint32_t dh = uint32_t(__double2hiint(kd));
-        largest = max(largest, dh & 0x7fffffffu);
-        const int ek = int(max(dh & 0x7fffffffu, oh & 0x7fffffffu) >> 20) - 1022;
-        const int sh = max(0, ek + 2 * (qz[k] - h) + 129);
-        const int bk = 893 - 2 * (qz[k] - h) + sh;
-        r.m[k][k] = fx_split(kd == 0.0 ? 0 : fx_from_words(dh, uint32_t(__double2loint(kd)), bk, 62));
+        const int sh = max(0, raw[k] - twice);
+        const int bk = 893 - 2 * (qz[k] - h) + sh + twice;
+        r.m[k][k] = fx_split((dh[k] << 1 | dl[k]) == 0 ? 0 : fx_from_words(dh[k], dl[k], bk, 62));
         r.m[1 - k][k] = fx_split(ko == 0.0 ? 0 : fx_from_words(oh, uint32_t(__double2loint(ko)), bk, 62));
         r.sh[k] = sh > 62 ? 63 : sh;  // past 62 every nonzero density goes the FP64 way
         r.q[k] = qz[k] + dq + 64 + fx_line_q(be, 62) - h;
@@ -648,7 +701,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       const FxRow& r = s_row[rho];
       const int4 pb = r.pb;
       const FxSplit m00 = r.m[0][0], m01 = r.m[0][1], m10 = r.m[1][0], m11 = r.m[1][1];
-      const int sh0 = r.sh[0], sh1 = r.sh[1];
+      const int sh0 = r.sh[0], sh1 = r.sh[1], twice = r.twice;
       const fx_t lim0 = fx_t(1) << max(0, 62 - sh0), lim1 = fx_t(1) << max(0, 62 - sh1);
       const bool diag = a.op.diag != 0, real = a.op.zi == 0.0;
       const int q0 = comp == 0 ? q : q_other, q1 = comp == 0 ? q_other : q;
@@ -673,16 +726,18 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
           int4 w0, w1;
           FxSplit g0, g1;
           if (real) {
-            g0 = fx_split(fx_expm1(f0));
-            g1 = fx_split(fx_expm1(f1));
+            fx_t e0 = fx_expm1(f0), e1 = fx_expm1(f1);
+            for (int k = 0; k < twice; ++k) {  // e^2x - 1 = 2 e + e^2
+              e0 = fx_mul(fx_split(e0), fx_split(e0), e0 << 1);
+              e1 = fx_mul(fx_split(e1), fx_split(e1), e1 << 1);
+            }
+            g0 = fx_split(e0);
+            g1 = fx_split(e1);
             z0 = fx_grow(x0, y0, z0, g0);
             z1 = fx_grow(x1, y1, z1, g1);
           } else {
-            fx_t sn, cm;
-            fx_sincos(f0, &sn, &cm);
-            w0 = fx_factor(cm, sn);
-            fx_sincos(f1, &sn, &cm);
-            w1 = fx_factor(cm, sn);
+            w0 = fx_phase(f0, twice);
+            w1 = fx_phase(f1, twice);
             z0 = fx_turn(x0, y0, z0, w0);
             z1 = fx_turn(x1, y1, z1, w1);
           }
@@ -702,7 +757,12 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
             z1 = fx_turn(x1, y1, z1, w1);
           }
         } else {
-          fx_point_far(&z0, &z1, q0, q1, dq, a.norm_num / s_w, a, x);
+          const double2 none = make_double2(0.0, 0.0);
+          const FxPair far = fx_point_far(
+              FxPair{z0, z1}, q0, q1, dq, a.norm_num / s_w, a.op.zr, a.op.zi, a.g_uu, a.g_dd, a.g_ud, a.op.m[0].p[x],
+              diag ? none : a.op.m[1].p[x], diag ? none : a.op.m[2].p[x], a.op.m[3].p[x]);
+          z0 = far.z0;
+          z1 = far.z1;
         }
         z0 = fx_cmul<false>(z0, pb);
         z1 = fx_cmul<false>(z1, pb);
@@ -755,9 +815,14 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
     }
   }
   int4* out = reinterpret_cast<int4*>(a.out[comp]);
-  const bool safe = fx_q_safe(q);
+  auto write = [&](auto form) {
 #pragma unroll
-  for (int m = 0; m < E; ++m) out[row_off + j + m * T] = bad ? fx_nan_words() : fx_words(v[0][m], q, safe);
+    for (int m = 0; m < E; ++m) out[row_off + j + m * T] = fx_words<decltype(form)::value, fx_convert(N, E)>(v[0][m], q);
+  };
+  const FxOut form = fx_out(bad, q);
+  if (form == kFxNear) write(std::integral_constant<FxOut, kFxNear>{});
+  else if (form == kFxBad) write(std::integral_constant<FxOut, kFxBad>{});
+  else write(std::integral_constant<FxOut, kFxFar>{});
 }
 
 template <int N, int E, int ROWS, int MINB>

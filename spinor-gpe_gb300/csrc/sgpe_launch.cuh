@@ -520,11 +520,14 @@ cudaError_t launch_col_grouped_s(const ColArgs<R>* args, int groups, int nx, int
   return dispatch_n(ny, ColGroupedLauncher<R, S>{args, groups, nx, s});
 }
 
-// Fixed-point complex128 passes: the tiles of the FP64 kernels' shapes at 64
-// registers (80 for the 12 points per thread of sides 3 * 2^k).  Measured at
-// 1024^2, step: 64 registers 400 us, 80 404 us, 128 422 us; at 768^2 80
-// registers 280 us, 64 435 us, 128 317 us.
-template <int E, int THREADS> constexpr int fx_minb() { return cmax(1, (E % 3 == 0 ? 768 : 1024) / THREADS); }
+// Fixed-point complex128 passes: the tiles of the FP64 kernels' shapes at 80
+// registers, 64 for 512-thread blocks (one of 80 leaves the SM half empty)
+// and for the 4 points per thread of the small shapes.  Measured, us a step,
+// 64 / 80 registers: 512^2 130.4 / 123.4, 768^2 435 / 280 (an earlier build),
+// 1024^2 411 / 407.5, 2048^2 1,750 / 2,152.
+template <int E, int THREADS> constexpr int fx_minb() {
+  return cmax(1, (E > 4 && THREADS <= 256 ? 768 : 1024) / THREADS);
+}
 
 template <int S> struct FxLauncher {
   const RowArgs<double>* row;   // one of the two passes
