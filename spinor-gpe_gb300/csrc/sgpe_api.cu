@@ -787,9 +787,25 @@ template <typename R> const sgpe::Cx<R>* cst(const void* p) { return static_cast
 
 // Fixed-point column operands of the kinetic factors applied (one or two
 // sets); without tables for one of them the FP64 kernels run.
+// Whether a sub-step of the plan turns (or damps) a state of the mean density
+// by more than 1/4 per interaction factor.  Most points of such a step are
+// past the series of the fixed-point rows and go their FP64 way one by one:
+// vortex grids (us a step, fixed point / FP64 passes) of 32^2 at 1.7 take 70.9
+// / 60.0, 64 x 32 at 0.86 74.0 / 62.7, 64^2 at 0.43 66.7 / 65.3, 128 x 64 at
+// 0.21 42.0 / 69.7.  The longest also amplify a rounding by 1e16 within 50
+// steps, so both directions keep the FP64 passes there and with them the bits.
+bool long_steps(const sgpe_plan* p) {
+  const double n = p->atom_num / (double(p->nx) * double(p->ny) * p->dv_r);
+  const double g = std::max({std::fabs(p->g[0]), std::fabs(p->g[1]), std::fabs(p->g[2])}) * n;
+  for (const SubOps& so : p->sub)
+    if (std::hypot(so.zr, so.zi) * g > 0.25) return true;
+  return false;
+}
+
 template <typename R> void col_fx(const sgpe_plan*, std::initializer_list<const SepOps*>, sgpe::ColArgs<R>*) {}
 template <>
 void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops, sgpe::ColArgs<double>* a) {
+  if (long_steps(p)) return;
   int i = 0;
   for (const SepOps* s : ops) {
     if (!s->fx_kin) return;
@@ -803,10 +819,11 @@ void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops
 }
 
 // Whether the row pass of sub-step `so` can run in fixed point: separable
-// operators with finite tables, an interaction factor that is a phase or
-// never above one (the point-wise results have no headroom to grow into).
+// operators with finite tables, no long steps, an interaction factor that is a
+// phase or never above one (the point-wise results have no headroom to grow
+// into).
 bool row_fx_ok(const sgpe_plan* p, const SubOps& so) {
-  if (p->bits != 128 || !fused_sep(so, p->coupling)) return false;
+  if (p->bits != 128 || !fused_sep(so, p->coupling) || long_steps(p)) return false;
   if (!(p->coupling ? so.sep.fx_c : so.sep.fx_d)) return false;
   if (so.zr == 0.0) return true;
   return so.zi == 0.0 && so.zr * p->g[0] <= 0.0 && so.zr * p->g[1] <= 0.0 && so.zr * p->g[2] <= 0.0;
@@ -821,13 +838,6 @@ template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowA
   for (int k = 0; k < 3; ++k) a->kz[k] = z * p->g[k];
   a->sqrt_norm = std::sqrt(a->norm_num);
   a->twf = static_cast<const int4*>(p->twf_x);
-}
-
-// The sums that the row pass of sub-step `sub` reads, or null when it adds up
-// the column pass's partials itself: the FP64 rows of a complex128 plan read
-// them (an FP64 sum of the partials in every row block costs them more).
-double* step_fin(const sgpe_plan* p, int sub) {
-  return p->final_sums || (p->bits == 128 && !row_fx_ok(p, p->sub[sub])) ? p->fin : nullptr;
 }
 
 // Column pass over the state (in place) ending a sub-step and starting `sub`.
@@ -870,7 +880,7 @@ template <typename R> bool col_step_args(sgpe_plan* p, int sub, bool want_u, sgp
   }
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
-  a.fin = step_fin(p, sub);
+  a.fin = p->final_sums ? p->fin : nullptr;
   a.count = p->count;
   return true;
 }
@@ -898,7 +908,7 @@ template <typename R> sgpe::RowArgs<R> row_step_args(sgpe_plan* p, int sub, doub
   a.scale = R(1);
   a.part = reinterpret_cast<R*>(p->part);
   a.ntile = p->ntile;
-  a.fin = step_fin(p, sub);
+  a.fin = p->final_sums ? p->fin : nullptr;
   a.norm_num = p->atom_num / (double(p->nx) * double(p->ny) * p->dv_r);
   a.g_uu = R(p->g[0]);
   a.g_dd = R(p->g[1]);
@@ -2240,7 +2250,7 @@ void build_groups(sgpe_batch* b) {
     auto fx = [](const sgpe_plan* q) {
       int n = 0;
       for (int sub = 0; sub < 2; ++sub) n += row_fx_ok(q, q->sub[sub]) ? 1 : 0;
-      for (int v = 0; v < 3; ++v) n += q->pair[v == 2][v == 1].sep.fx_kin ? 1 : 0;
+      for (int v = 0; v < 3; ++v) n += q->pair[v == 2][v == 1].sep.fx_kin && !long_steps(q) ? 1 : 0;
       return n == 5 ? 1 : n == 0 ? 0 : -1;
     };
     if (!b->grouping || !sep(p) || fx(p) < 0) continue;

@@ -468,6 +468,25 @@ __device__ __forceinline__ FloatFloat sum_partials_w(const float* part, int ntil
   return sw;
 }
 
+// ... and of FP64 partials.
+__device__ __forceinline__ double sum_partials_w(const double* part, int ntile, int lane) {
+  double sw = 0.0;
+  for (int i0 = lane; i0 < 2 * ntile; i0 += 32 * kPartialBatch) {
+    double v[kPartialBatch];
+#pragma unroll
+    for (int k = 0; k < kPartialBatch; ++k) {
+      const int i = i0 + 32 * k;
+      v[k] = i < 2 * ntile ? part[2 * i + 1] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPartialBatch; ++k) {
+      if (i0 + 32 * k >= 2 * ntile) break;
+      sw += v[k];
+    }
+  }
+  return warp_sum(sw);
+}
+
 // lambda = sqrt(num / w) of the row pass, in the working precision.  Warp 0
 // of every row block sums the partials while the block waits at the barrier
 // in front of the point-wise step, so the population sums are formed only
@@ -486,9 +505,13 @@ __device__ __forceinline__ float row_lambda(const float* part, int ntile, int la
   return sqrtf(norm_num / (c.hi + c.lo));
 }
 __device__ __forceinline__ double row_lambda(const double* part, int ntile, int lane, double norm_num, double* u0,
-                                             double* u1, bool) {
+                                             double* u1, bool want_u) {
   double sw;
-  sum_partials(part, ntile, lane, u0, u1, &sw);
+  if (want_u) {
+    sum_partials(part, ntile, lane, u0, u1, &sw);
+  } else {
+    sw = sum_partials_w(part, ntile, lane);
+  }
   return sqrt(norm_num / sw);
 }
 // double-float: the sums in double-float, the square root of the quotient in

@@ -112,6 +112,19 @@ def test_steps_match_oracle(tp, tmp_path, nx, ny, time, dt, g, omega):
     np.testing.assert_allclose(pops.cpu().numpy(), ref_pops, rtol=1e-12, atol=1e-13)
 
 
+# one step on either side of the longest that runs in fixed point: 1/4 rad (or
+# e-folding) per interaction factor at the mean density, here 3.016 dt
+@pytest.mark.parametrize('time', ['real', 'imag'])
+@pytest.mark.parametrize('dt', [0.01, 0.04, 0.0796, 0.0862, 0.3])
+def test_longest_steps_match_oracle(tp, tmp_path, time, dt):
+    ps = _problem(tmp_path, 64, 64, (1000.0, 995.0, 990.0), 0.7, delta=0.3)
+    ref, _ = _oracle(ps, dt, time, 1)
+    prop = tp.TensorPropagator(ps, dt, 1, 'cuda', time=time, dtype=128)
+    prop.full_steps(1)
+    got = np.array([t.cpu().numpy() for t in prop.psik])
+    assert rel_l2(got, ref) <= 1e-12
+
+
 @pytest.mark.parametrize('amp', [1e-9, 0.0])
 def test_minority_component_keeps_its_precision(tp, tmp_path, amp):
     ps = _problem(tmp_path, 128, 64, (1000.0, 995.0, 990.0), None)
