@@ -785,8 +785,6 @@ template <typename R> sgpe::RealOp<R> real_op(const SubOps& so, int coupling) {
 template <typename R> sgpe::Cx<R>* st(void* p) { return static_cast<sgpe::Cx<R>*>(p); }
 template <typename R> const sgpe::Cx<R>* cst(const void* p) { return static_cast<const sgpe::Cx<R>*>(p); }
 
-// Fixed-point column operands of the kinetic factors applied (one or two
-// sets); without tables for one of them the FP64 kernels run.
 // Whether a sub-step of the plan turns (or damps) a state of the mean density
 // by more than 1/4 per interaction factor.  Most points of such a step are
 // past the series of the fixed-point rows and go their FP64 way one by one:
@@ -802,6 +800,8 @@ bool long_steps(const sgpe_plan* p) {
   return false;
 }
 
+// Fixed-point column operands of the kinetic factors applied (one or two
+// sets); without tables for one of them the FP64 kernels run.
 template <typename R> void col_fx(const sgpe_plan*, std::initializer_list<const SepOps*>, sgpe::ColArgs<R>*) {}
 template <>
 void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops, sgpe::ColArgs<double>* a) {

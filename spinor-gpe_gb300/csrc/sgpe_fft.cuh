@@ -536,6 +536,22 @@ __host__ __device__ constexpr int tw_offset(int N, int E, int NS) {
   return off;
 }
 
+// Elements of `bytes` bytes from one column's exchange line to the next where
+// the threads of a warp walk `cols` columns side by side (lane l: column l %
+// cols).  A warp's shared-memory access of 8- or 16-byte elements is served 16
+// or 8 lanes at a time, one per bank group: those lanes hold every column and
+// `step` neighbouring elements of each, so an odd multiple of `step` puts the
+// columns' elements side by side in the banks.  (A fixed pad of 2 does so only
+// for 8 columns of complex64 and 4 of 16 bytes; with 4 and 2 columns 45% of
+// the column pass's wavefronts were conflicts: a pass of complex64 4096^2 312
+// -> 265 us, complex128 1024^2 64.3 -> 60.6, double-float 2048^2 279 -> 267.)
+__host__ __device__ constexpr int column_line_stride(int n, int e, int cols, int bytes) {
+  const int step = 128 / bytes > cols ? 128 / bytes / cols : 1;
+  int s = n + n / e;
+  while (cols > 1 && s % (2 * step) != step) ++s;
+  return s;
+}
+
 // Shared-memory view used by the exchange stages: element i of line l of the
 // calling thread's group lives at base[l * line_stride + i + i / E] (one pad
 // element per E elements keeps the radix-E scatter free of bank conflicts).

@@ -231,7 +231,7 @@ template <int NW, int COLS> __device__ __forceinline__ uint32_t fx_max_entries(c
 template <int N, int E, int COLS>
 __device__ __forceinline__ void col_body_fx(const ColArgs<double>& a, const BlockPos pos) {
   constexpr int T = N / E;
-  constexpr int LS = N + N / E + 2;
+  constexpr int LS = column_line_stride(N, E, COLS, sizeof(FxC));
   constexpr int NT = T * COLS;
   constexpr int NW = NT / 32;
   constexpr int kBits = fx_bits(stage_radix(N, E, 1));

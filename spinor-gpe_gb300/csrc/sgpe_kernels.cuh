@@ -1074,7 +1074,7 @@ __device__ __forceinline__ void col_body(const ColArgs<R>& a, const BlockPos pos
   using C = Cx<R>;
   static_assert(!TC || sizeof(R) == 4, "tensor-core DFT16 is complex64 only");
   constexpr int T = N / E;
-  constexpr int LS = N + N / E + 2;
+  constexpr int LS = column_line_stride(N, E, COLS, sizeof(C));
   constexpr int NT = T * COLS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
@@ -1101,7 +1101,7 @@ __device__ __forceinline__ void col_body(const ColArgs<R>& a, const BlockPos pos
   constexpr bool kTma = SGPE_COL_TMA && N >= SGPE_COL_TMA_MIN_N && !QUEUE;
   constexpr int kBoxY = N < 256 ? N : 256;
   constexpr uint32_t kTileBytes = uint32_t(COLS) * N * sizeof(C);
-  static_assert(!kTma || sizeof(C) * COLS * (N / E + 2) >= 128, "the aligned tile must fit the exchange area");
+  static_assert(!kTma || sizeof(C) * COLS * (LS - N) >= 128, "the aligned tile must fit the exchange area");
   static_assert(!kTma || (COLS * sizeof(C)) % 16 == 0, "tile rows must be whole 16-byte units");
   C* const stage = reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const char* const tmap = static_cast<const char*>(a.tmap) + comp * 128;

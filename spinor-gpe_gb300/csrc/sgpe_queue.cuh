@@ -69,7 +69,7 @@ template <int N> struct QueueShape {
   static constexpr int ROWS = kQueueThreads / (2 * T);
   static constexpr int COLS = kQueueThreads / T;
   static constexpr size_t ROW_SMEM = 2ull * ROWS * (N + N / E) * sizeof(float2);
-  static constexpr size_t COL_SMEM = size_t(COLS) * (N + N / E + 2) * sizeof(float2);
+  static constexpr size_t COL_SMEM = sizeof(float2) * COLS * column_line_stride(N, E, COLS, sizeof(float2));
   static_assert(ROWS >= 1 && COLS >= 1 && 2 * T * ROWS == kQueueThreads && T * COLS == kQueueThreads,
                 "queue items fill the block");
 };
