@@ -397,6 +397,18 @@ int default_shape(int bits, int axis, int n) {
   return 0;
 }
 
+// Column shape of a plan.  complex64 columns of 2048 run in tiles of 8 columns
+// (one 1024-thread block per SM) or of 4 (two of 512, one loading while the
+// other transforms).  The pair is no faster than the large block where a wave
+// ends with both halves of most SMs taken, so the tiles of 4 are for widths
+// whose last wave fills at most half of the 304 places: us a step, 8 / 4
+// columns, nx = 256: 75.4 / 59.3, 768: 158 / 145, 2048: 317 / 305; against
+// 384: 96.0 / 100.7, 512: 92.2 / 95.2, 1024: 166.7 / 170.0.
+int default_col_shape(int bits, int nx, int ny) {
+  if (bits == 64 && ny == 2048) return (nx / 2) % 304 <= 152 ? 1 : 0;
+  return default_shape(bits, 1, ny);
+}
+
 int shape_count(int bits, int axis, int n) {
   if (!sgpe::size_supported(n)) return 0;
   if (bits == 64) return axis == 0 ? sgpe::row_shape_count<float>(n) : sgpe::col_shape_count<float>(n);
@@ -1445,7 +1457,7 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
   const char* fs = std::getenv("SGPE_FINAL_SUMS");
   p->final_sums = fs != nullptr ? fs[0] == '1' : dtype_bits == SGPE_DTYPE_DF || (dtype_bits == 128 && nx >= 2048);
   p->row_shape = default_shape(dtype_bits, 0, nx);
-  p->col_shape = default_shape(dtype_bits, 1, ny);
+  p->col_shape = default_col_shape(dtype_bits, nx, ny);
   int cols = by_prec(dtype_bits, [&](auto t) { return sgpe::col_tile_width<decltype(t)>(ny, p->col_shape); });
   if (cols == 0 || nx % cols != 0 || (nx / 2) % cols != 0) {
     // the default shape's tile does not divide nx: shape 0

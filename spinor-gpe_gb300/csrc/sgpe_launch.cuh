@@ -167,12 +167,14 @@ template <> struct ShapeTune<float> {
   static constexpr int row_shapes(int n) {
     return n % 3 == 0 ? 2 : !is_pow2(n) ? 1 : n <= 512 ? 3 : n == 1024 ? 2 : 1;
   }
-  static constexpr int col_shapes(int n) { return n % 3 == 0 ? 2 : (is_pow2(n) && n <= 512) ? 3 : 1; }
+  // columns: 8 points per thread up to 512 (shape 2 in tiles of 4); 2048 with
+  // 16 in tiles of 4 (default_col_shape)
+  static constexpr int col_shapes(int n) { return n % 3 == 0 || n == 2048 ? 2 : (is_pow2(n) && n <= 512) ? 3 : 1; }
   static constexpr int row_e(int n, int s) { return n % 3 == 0 ? r3_alt(n) : n == 1024 ? 32 : s == 1 ? 8 : 4; }
   static constexpr int row_minb(int n, int) { return n == 1024 ? 4 : 0; }  // 0: the shape-0 rule
   static constexpr int row_threads(int, int) { return Tune<float>::ROW_THREADS; }
-  static constexpr int col_e(int n, int) { return n % 3 == 0 ? r3_alt(n) : 8; }
-  static constexpr int cols(int n, int s) { return (n % 3 != 0 && s == 2) ? 4 : Tune<float>::COLS; }
+  static constexpr int col_e(int n, int) { return n % 3 == 0 ? r3_alt(n) : n == 2048 ? 16 : 8; }
+  static constexpr int cols(int n, int s) { return n == 2048 || (n % 3 != 0 && s == 2) ? 4 : Tune<float>::COLS; }
 };
 // complex128: 4 points per thread up to 512; shape 2 also halves the lines
 // per block (128-thread row blocks, 2-column tiles of 32-byte row segments),

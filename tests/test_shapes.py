@@ -357,3 +357,23 @@ def test_batch_autotune_keeps_states_and_matches_solves_alone(tp, tmp_path):
         a.full_steps(13)
         np.testing.assert_array_equal(_psik(a), _psik(p))
     batch.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('nx', [32, 256, 384])
+def test_columns_of_2048_in_both_tiles(tmp_path, nx):
+    """Tiles of 8 and of 4 columns; the default by the width's last wave."""
+    from test_fixed_point import _oracle, _problem
+    from spinor_gpe.pspinor import tensor_propagator as tp
+    ps = _problem(tmp_path, nx, 2048, (1000.0, 995.0, 990.0), 1.0)
+    ref, _ = _oracle(ps, 1e-3, 'real', 2)
+    prop = tp.TensorPropagator(ps, 1e-3, 2, 'cuda', time='real', dtype=64)
+    row, col = prop.kernel_shapes
+    assert col == (0 if nx == 384 else 1)
+    psik = [p.clone() for p in prop.psik]
+    for shape in (col, 1 - col):
+        prop.kernel_shapes = (row, shape)
+        prop.psik = psik
+        prop.full_steps(2)
+        got = np.array([t.cpu().numpy() for t in prop.psik])
+        assert rel_l2(got, ref) <= 1e-5
