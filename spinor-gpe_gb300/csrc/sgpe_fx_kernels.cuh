@@ -4,14 +4,13 @@
 // sums on them, and writes FP64 again.  Same passes, arguments and tiles as
 // col_body / row_body.
 //
-// Bound: integer issue.  At 1024^2 a column pass issues about 530
-// instructions per point and component (93 of them multiply-adds at 2.6
-// cycles) and a row pass 750, at two instructions per cycle and SM
-// sub-partition pair; DRAM and L2 are under 15% busy.  Measured at 1024^2
-// (real time, Raman coupling; column / row / step): FP64 butterflies 347 /
-// 473 / 2,470 us, fixed point 69 / 85 / 425 us, with the error against 64
-// bits unchanged or smaller (8 steps, 256^2 to 4096 x 128: 0.6-1.3 of the
-// FP64 kernels', geometric mean 0.87).
+// Bound: integer issue.  At 1024^2 a column pass issues 511 instructions per
+// point and component (wide multiply-adds take their pipe for 2-2.6 cycles)
+// and a row pass 754, at two instructions per cycle and SM; DRAM and L2 are
+// under 15% busy.  Measured at 1024^2 (real time, Raman coupling; column / row
+// / step): FP64 butterflies 347 / 473 / 2,470 us, fixed point 60.6 / 83.3 /
+// 400 us, with the error against 64 bits on average smaller (8 steps of six
+// problems, 64^2 to 4096 x 128: geometric mean 0.87 of the FP64 kernels').
 #pragma once
 #include "sgpe_kernels.cuh"
 
