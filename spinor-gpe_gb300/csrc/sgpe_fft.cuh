@@ -657,14 +657,20 @@ __device__ __forceinline__ void fft_stage(C (&v)[L][E], int j, const SM& sm, con
           a[l][q][r] = FxC{a[l][q][r].x << sm.pre, a[l][q][r].y << sm.pre};
       }
   if constexpr (is_fx<C>::value && kLast && !kFirst) {
-    // room that the line's values left in front of the last stage
+    // room that the line's values left in front of the last stage (missing
+    // room is rare: a branch costs the others nothing)
     const int up = sm.up();
+    auto shift = [&](auto down) {
 #pragma unroll
-    for (int l = 0; l < L; ++l)
+      for (int l = 0; l < L; ++l)
 #pragma unroll
-      for (int q = 0; q < Q; ++q)
+        for (int q = 0; q < Q; ++q)
 #pragma unroll
-        for (int r = 0; r < R; ++r) a[l][q][r] = FxC{a[l][q][r].x << up, a[l][q][r].y << up};
+          for (int r = 0; r < R; ++r)
+            a[l][q][r] = decltype(down)::value ? fx_shift(a[l][q][r], up) : FxC{a[l][q][r].x << up, a[l][q][r].y << up};
+    };
+    if (up >= 0) shift(std::false_type{});
+    else shift(std::true_type{});
   }
   if constexpr (!kFirst && SGPE_TW_FACTOR && Q > 1 && T * Q == NS) {
     // The Q butterflies of the thread sit at k = j + qT with NS = TQ, so

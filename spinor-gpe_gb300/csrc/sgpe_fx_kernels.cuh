@@ -28,6 +28,12 @@ template <int N, int E, bool LAST = true> __host__ __device__ constexpr int fx_t
   return q;
 }
 
+__host__ __device__ constexpr int last_radix(int n, int e) {
+  int ns = 1, r = 1;
+  while (ns < n) ns *= r = stage_radix(n, e, ns);
+  return r;
+}
+
 // A thread's share of its line's L1 norm in units of 2^44, rounded up: the
 // high words' magnitudes fit 32 bits for |z| < 2^(62.5 - bits(E)).
 template <int E> __device__ __forceinline__ uint32_t fx_l1(const FxC (&v)[E]) {
@@ -76,9 +82,10 @@ template <int N, int E, bool WARP, bool PAIR> struct FxLine : LineSmem<FxC, E, W
     }
     if (PAIR && common) s = t = max(s, t);
     constexpr int kScaled = fx_transform_q<N, E, false>();
-    const int u = fx_room(s, kScaled - pre);
+    constexpr int kLastRadix = last_radix(N, E);
+    const int u = fx_room(s, kScaled - pre, kLastRadix);
     shift = u + pre;
-    if (PAIR) shift_other = fx_room(t, kScaled);
+    if (PAIR) shift_other = fx_room(t, kScaled, kLastRadix);
     return u;
   }
 };

@@ -57,6 +57,43 @@ def test_transforms_of_peaks_zeros_and_nan(shape):
         assert not got[1].any()
 
 
+# a line whose values all add up in one bin, with parts that fill their
+# exponent (1.9 +- 1.9i in four domains of constant phase): the largest sums a
+# transform can meet
+@pytest.mark.parametrize('side', [32, 64, 128, 192, 256, 384, 512, 768, 1024, 2048, 4096])
+def test_transforms_of_full_lines(side):
+    from spinor_gpe.pspinor import tensor_tools as ttools
+    line = (1.9 + 1.9j) * 1j**(np.arange(side) * 4 // side)
+    for shape, field in (((32, side), np.ones((32, 1)) * line), ((side, 32), line[:, None] * np.ones(32))):
+        psi = [field, np.roll(field, 3, (0, 1)).conj()]
+        got = ttools.fft_2d([torch.as_tensor(p, device='cuda') for p in psi], (1.0, 2 * np.pi))
+        back = ttools.ifft_2d([torch.as_tensor(np.fft.fftshift(p), device='cuda') for p in psi], (1.0, 2 * np.pi))
+        for g, b, p in zip(got, back, psi):
+            assert rel_l2(g.cpu().numpy(), np.fft.fftshift(np.fft.fftn(p))) <= 8e-15
+            assert rel_l2(b.cpu().numpy(), np.fft.ifftn(p)) <= 8e-15
+
+
+# steps of states that are such lines in k space (flat spectra, whose rows add
+# up in one point): a point in real space, and the four domains along kx and ky
+@pytest.mark.parametrize('state', ['point', 'domains'])
+@pytest.mark.parametrize('nx,ny', [(64, 512), (512, 64), (32, 32), (1024, 128), (64, 1024)])
+def test_steps_of_full_lines_match_oracle(tp, tmp_path, nx, ny, state):
+    ps = _problem(tmp_path, nx, ny, (1000.0, 995.0, 990.0), 0.7)
+    ps.g_sc = {'uu': 1e-3, 'dd': 1e-3, 'ud': 1e-3}
+    if state == 'point':
+        psi = np.zeros((ny, nx), dtype=complex)
+        psi[ny // 2, nx // 2] = 1.0
+        psi = np.fft.fftshift(np.fft.fft2(psi))
+    else:
+        psi = (1.9 + 1.9j) * 1j**(np.arange(nx) * 4 // nx) * 1j**(np.arange(ny) * 4 // ny)[:, None]
+    ps.psik = [psi, 0.9 * psi.conj()]
+    ref, _ = _oracle(ps, 1e-3, 'real', 2)
+    prop = tp.TensorPropagator(ps, 1e-3, 2, 'cuda', time='real', dtype=128)
+    prop.full_steps(2)
+    got = np.array([t.cpu().numpy() for t in prop.psik])
+    assert rel_l2(got, ref) <= 1e-12
+
+
 def _problem(tmp_path, nx, ny, g, omega, dtype=np.complex128, **kw):
     from spinor_gpe import workloads
     from spinor_gpe.pspinor import pspinor as spin
