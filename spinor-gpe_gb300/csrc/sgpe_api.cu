@@ -339,7 +339,7 @@ int upload_int4(const std::vector<int4>& h, void** out, std::vector<void*>* allo
 }
 
 // Twiddle table of an (n, e) transform in fixed point: the entries of
-// upload_twiddles times 2^(64 - fx_stage_bits) (sgpe_fx.cuh).  The roots of
+// upload_twiddles times 2^(64 - fx_bits) (sgpe_fx.cuh).  The roots of
 // order n are products of two short tables evaluated in extended precision,
 // rounded at 2^-62 (evaluating every root so took 2 ms a plan).
 int upload_twiddles_fx(int n, int e, void** out) {
@@ -363,7 +363,7 @@ int upload_twiddles_fx(int n, int e, void** out) {
   for (int ns = 1; ns < n;) {
     const int rs = sgpe::stage_radix(n, e, ns);
     const int len = ns * rs;
-    const int down = 60 + sgpe::fx_stage_bits(rs, len == n);  // 2^124 -> 2^(64 - bits)
+    const int down = 60 + sgpe::fx_bits(rs);  // 2^124 -> 2^(64 - bits)
     for (int r = 1; r < rs; ++r)
       for (int k = 0; k < ns; ++k) {
         const int m = int(((long long)k * r) % len) * (n / len);

@@ -657,20 +657,14 @@ __device__ __forceinline__ void fft_stage(C (&v)[L][E], int j, const SM& sm, con
           a[l][q][r] = FxC{a[l][q][r].x << sm.pre, a[l][q][r].y << sm.pre};
       }
   if constexpr (is_fx<C>::value && kLast && !kFirst) {
-    // room that the line's values left in front of the last stage (missing
-    // room is rare: a branch costs the others nothing)
+    // room that the line's values left in front of the last stage
     const int up = sm.up();
-    auto shift = [&](auto down) {
 #pragma unroll
-      for (int l = 0; l < L; ++l)
+    for (int l = 0; l < L; ++l)
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
+      for (int q = 0; q < Q; ++q)
 #pragma unroll
-          for (int r = 0; r < R; ++r)
-            a[l][q][r] = decltype(down)::value ? fx_shift(a[l][q][r], up) : FxC{a[l][q][r].x << up, a[l][q][r].y << up};
-    };
-    if (up >= 0) shift(std::false_type{});
-    else shift(std::true_type{});
+        for (int r = 0; r < R; ++r) a[l][q][r] = FxC{a[l][q][r].x << up, a[l][q][r].y << up};
   }
   if constexpr (!kFirst && SGPE_TW_FACTOR && Q > 1 && T * Q == NS) {
     // The Q butterflies of the thread sit at k = j + qT with NS = TQ, so
@@ -698,7 +692,7 @@ __device__ __forceinline__ void fft_stage(C (&v)[L][E], int j, const SM& sm, con
       const W* twq = reinterpret_cast<const W*>(tw) + kOff + (vt % NS);
       if constexpr (is_fx<C>::value) {  // the factor one, with the stage's scaling
 #pragma unroll
-        for (int l = 0; l < L; ++l) a[l][q][0] = fx_scale_down<fx_stage_bits(R, kLast)>(a[l][q][0]);
+        for (int l = 0; l < L; ++l) a[l][q][0] = fx_scale_down<fx_bits(R)>(a[l][q][0]);
       }
 #pragma unroll
       for (int r = 1; r < R; ++r) {

@@ -12,13 +12,13 @@
 // its first stage with |z| < 2^(62.5 - bits(R)), bits(R) = max(2, ceil log2
 // R), and the twiddles of every later stage carry the factor 2^-bits(R); no
 // sum can leave 63 bits, whatever the data.  That scaling assumes values that
-// all add up.  No partial sum of a transform exceeds the line's sum of
-// |re| + |im| (its L1 norm), which is much less for a spectrum of a few lines
-// or a cloud in a large box, so the line is shifted in front of its last
-// stage to what its L1 norm leaves free (fx_room), and that stage's twiddles
-// carry 2^-2 whatever its radix.  The shift is down, by up to
-// log2 R bits, for a line whose values do add up (a line of 512 in four
-// domains of constant phase would reach 2^63.3 in a last radix 8).
+// all add up (a spectrum of unit modulus, domains of constant phase).  No
+// partial sum of a transform exceeds the line's sum of |re| + |im| (its L1
+// norm), which is much less for a spectrum of a few lines or a cloud in a
+// large box, so the line is shifted up in front of its last stage by what its
+// L1 norm leaves free (fx_room).  Behind a transform either every |z| is
+// below 2^60.5 (its L1 norm had room), or their root sum square is below
+// 2^62.5 (that of a line whose values all add up is its largest sum).
 //
 // Precision: a product is rounded within 0.6 units and a line's values come
 // in at 2^-59 of its largest.
@@ -113,21 +113,17 @@ __host__ __device__ constexpr int fx_bits(int radix) {
   return b;
 }
 
-// Bits free (negative: missing) in front of the last stage of a line whose L1
-// norm is below l1 2^44, after stages that scaled it by 2^-scaled: with the
-// norm there below 2^62, the last stage's results stay below 2^60.  Without
-// the norm (which counts 2^44 a thread for values below that) no value is above
-// 2^62.5 and a shift by -ceil log2 R keeps the results below 2^60.5.
-__host__ __device__ __forceinline__ int fx_room(uint32_t l1, int scaled, int radix) {
+// Bits free in front of the last stage of a line whose L1 norm is below
+// l1 2^44, after stages that scaled it by 2^-scaled: the values there may be
+// shifted up to 2^62.
+__host__ __device__ __forceinline__ int fx_room(uint32_t l1, int scaled) {
 #ifdef __CUDA_ARCH__
   const int b = 32 - __clz(int(l1));
 #else
   const int b = l1 ? 32 - __builtin_clz(l1) : 0;
 #endif
-  int least = 0;
-  while ((1 << least) < radix) ++least;
   const int up = 62 - 44 - b + scaled;
-  return up > -least ? up : -least;
+  return up > 0 ? up : 0;
 }
 
 // a 2^-B, rounded
@@ -135,16 +131,6 @@ template <int B> __host__ __device__ __forceinline__ FxC fx_scale_down(FxC a) {
   const fx_t half = fx_t(1) << (B - 1);
   return FxC{(a.x + half) >> B, (a.y + half) >> B};
 }
-
-// a 2^up, rounded, up of either sign
-__host__ __device__ __forceinline__ FxC fx_shift(FxC a, int up) {
-  if (up >= 0) return FxC{a.x << up, a.y << up};
-  const fx_t half = fx_t(1) << (-up - 1);
-  return FxC{(a.x + half) >> -up, (a.y + half) >> -up};
-}
-
-// bits a stage's twiddles scale by
-__host__ __device__ constexpr int fx_stage_bits(int radix, bool last) { return last ? 2 : fx_bits(radix); }
 
 // ------------------------------------------------ FP64 <-> fixed point
 __host__ __device__ __forceinline__ uint64_t fx_shr(uint64_t m, int d) {  // d >= 0; 0 from 64 on

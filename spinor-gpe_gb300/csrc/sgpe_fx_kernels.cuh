@@ -22,16 +22,10 @@ template <int N, int E, bool LAST = true> __host__ __device__ constexpr int fx_t
   int q = 0, ns = stage_radix(N, E, 1);
   while (ns < N) {
     const int r = stage_radix(N, E, ns);
-    if (LAST || ns * r < N) q += fx_stage_bits(r, ns * r == N);
+    if (LAST || ns * r < N) q += fx_bits(r);
     ns *= r;
   }
   return q;
-}
-
-__host__ __device__ constexpr int last_radix(int n, int e) {
-  int ns = 1, r = 1;
-  while (ns < n) ns *= r = stage_radix(n, e, ns);
-  return r;
 }
 
 // A thread's share of its line's L1 norm in units of 2^44, rounded up: the
@@ -82,10 +76,9 @@ template <int N, int E, bool WARP, bool PAIR> struct FxLine : LineSmem<FxC, E, W
     }
     if (PAIR && common) s = t = max(s, t);
     constexpr int kScaled = fx_transform_q<N, E, false>();
-    constexpr int kLastRadix = last_radix(N, E);
-    const int u = fx_room(s, kScaled - pre, kLastRadix);
+    const int u = fx_room(s, kScaled - pre);
     shift = u + pre;
-    if (PAIR) shift_other = fx_room(t, kScaled, kLastRadix);
+    if (PAIR) shift_other = fx_room(t, kScaled);
     return u;
   }
 };
@@ -648,9 +641,10 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       const double px = mb.x * lam, py = mb.y * lam;
       const uint32_t xh = uint32_t(__double2hiint(px)), yh = uint32_t(__double2hiint(py));
       const int be = fx_line_exp(max(xh & 0x7fffffffu, yh & 0x7fffffffu));
-      // |z| <= 2^60.5 (the last stage scales by at least 2^-2), a quarter of
-      // it behind the matrix: a factor of up to 2^62.5 leaves the headroom of
-      // any first stage
+      // |z| <= 2^60.5, half of it (two products of a quarter) behind the
+      // matrix: a factor of up to 2^62.5 leaves the headroom of any first
+      // stage; a root sum square of 2^62.5 becomes 2^60, of which R points of
+      // a butterfly add up to sqrt(R) 2^60
       r.pb = fx_factor(fx_from_words(xh, uint32_t(__double2loint(px)), be, 62),
                        fx_from_words(yh, uint32_t(__double2loint(py)), be, 62));
       const int qz[2] = {q, q_other};
