@@ -76,9 +76,10 @@ struct SepOps {
   // (sgpe_fx.cuh), times 2^-exponent; not made when a table holds a value
   // that is not finite
   void* fky[2] = {nullptr, nullptr};
-  void* fm = nullptr;    // m[0..3] one after the other
+  void* fm = nullptr;    // m[0..3] one after the other, with one exponent
+  void* fms = nullptr;   // ... with an exponent each
   void* fdg = nullptr;   // dg[0..1]
-  int fke[2] = {0, 0}, fme = 0, fdge = 0;
+  int fke[2] = {0, 0}, fme = 0, fmse[4] = {0, 0, 0, 0}, fdge[2] = {0, 0};
   bool fx_kin = false, fx_c = false, fx_d = false;
 };
 
@@ -561,6 +562,9 @@ HostField host_field(const sgpe_field& f) {
   return h;
 }
 
+// Exponent of a table of zeros: below any sum it can be a term of.
+constexpr int kFxZeroTable = -4096;
+
 // Smallest e with every |value| of the fields at most 2^e (to rounding);
 // false when a value is not finite.
 bool fx_exponent(std::initializer_list<const HostField*> fields, int* e) {
@@ -571,18 +575,20 @@ bool fx_exponent(std::initializer_list<const HostField*> fields, int* e) {
       if (!std::isfinite(m)) return false;
       most = std::max(most, m);
     }
-  *e = 0;
+  *e = kFxZeroTable;
   if (most > 0.0) std::frexp(most * (1.0 - 1e-9), e);
   return true;
 }
 
-// Tables of equal length as split fixed-point factors, value 2^(62 - e), one
-// after the other.
-int upload_fx(std::initializer_list<const HostField*> fields, int e, void** out, std::vector<void*>* allocs) {
+// Tables of equal length as split fixed-point factors, value 2^(62 - e) (e of
+// each table), one after the other.
+int upload_fx(std::initializer_list<const HostField*> fields, const int* e, void** out, std::vector<void*>* allocs) {
   std::vector<int4> h;
-  for (const HostField* f : fields)
+  for (const HostField* f : fields) {
     for (size_t i = 0; i < f->v.size(); i += 2)
-      h.push_back(fx_entry(std::llrint(std::ldexp(f->v[i], 62 - e)), std::llrint(std::ldexp(f->v[i + 1], 62 - e))));
+      h.push_back(fx_entry(std::llrint(std::ldexp(f->v[i], 62 - *e)), std::llrint(std::ldexp(f->v[i + 1], 62 - *e))));
+    ++e;
+  }
   return upload_int4(h, out, allocs, "fixed-point table");
 }
 
@@ -602,7 +608,7 @@ int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2]
   for (int c = 0; c < 2; ++c) {
     int ex = 0;
     if (!fx_exponent({&x[c]}, &ex) || !fx_exponent({&y[c]}, &so->fke[c])) return SGPE_OK;
-    const int rc = upload_fx({&y[c]}, so->fke[c], &so->fky[c], allocs);
+    const int rc = upload_fx({&y[c]}, &so->fke[c], &so->fky[c], allocs);
     if (rc != SGPE_OK) return rc;
   }
   so->fx_kin = true;
@@ -662,7 +668,7 @@ int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2]
   so->mb_real = imag_zero(py[0]);
   so->fused_d = true;
   const bool fx = p->bits == 128;
-  if (fx && fx_exponent({&dg[0], &dg[1]}, &so->fdge)) {
+  if (fx && fx_exponent({&dg[0]}, &so->fdge[0]) && fx_exponent({&dg[1]}, &so->fdge[1])) {
     rc = upload_fx({&dg[0], &dg[1]}, so->fdge, &so->fdg, allocs);
     if (rc != SGPE_OK) return rc;
     so->fx_d = true;
@@ -672,7 +678,10 @@ int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2]
     if (rc != SGPE_OK) return rc;
     so->fused_c = true;
     if (fx && fx_exponent({&m[0], &m[1], &m[2], &m[3]}, &so->fme)) {
-      rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, so->fme, &so->fm, allocs);
+      for (int k = 0; k < 4; ++k) fx_exponent({&m[k]}, &so->fmse[k]);
+      const int one[4] = {so->fme, so->fme, so->fme, so->fme};
+      rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, one, &so->fm, allocs);
+      if (rc == SGPE_OK) rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, so->fmse, &so->fms, allocs);
       if (rc != SGPE_OK) return rc;
       so->fx_c = true;
     }
@@ -847,8 +856,13 @@ template <typename R> void row_fx(const sgpe_plan*, const SubOps&, sgpe::RowArgs
 template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowArgs<double>* a) {
   if (!row_fx_ok(p, so)) return;
   const int4* m = static_cast<const int4*>(p->coupling ? so.sep.fm : so.sep.fdg);
-  for (int k = 0; k < 4; ++k) a->mf[k] = m + (p->coupling ? k : k / 2) * p->nx;
-  a->me = p->coupling ? so.sep.fme : so.sep.fdge;
+  for (int k = 0; k < 4; ++k) {
+    a->mf[k] = m + (p->coupling ? k : k / 2) * p->nx;
+    a->me[k] = p->coupling ? so.sep.fme : so.sep.fdge[k / 2];
+    a->ms[k] = p->coupling ? static_cast<const int4*>(so.sep.fms) + k * p->nx : nullptr;
+    a->mse[k] = so.sep.fmse[k];
+  }
+  a->split = std::abs(std::max(a->mse[0], a->mse[1]) - std::max(a->mse[2], a->mse[3])) > sgpe::kFxUnlike;
   const double z = (so.zi != 0.0 ? so.zi : so.zr) * a->norm_num;
   for (int k = 0; k < 3; ++k) a->kz[k] = z * p->g[k];
   a->sqrt_norm = std::sqrt(a->norm_num);

@@ -51,10 +51,18 @@ __device__ __forceinline__ int fx_pre(uint32_t largest, int bits) {
   return max(0, min(__clz(int(largest + 1)) - 2 - bits, 24));
 }
 
+// Components that a coupling mixes are held at one exponent where theirs are
+// at most this far apart (of 59 bits two go), and at their own where they are
+// further: a polarised gas under a weak drive keeps the bits of its minority
+// (two steps from 1e-6 of the other's amplitude at omega = 1e-3: 7e-11 of
+// itself with one exponent, 4e-16 so).
+constexpr int kFxUnlike = 2;
+
 // The exchange lines of a fixed-point transform.  A line's L1 norm is what
 // its threads know (own) plus `warps` entries in shared memory, written in
 // front of the transform's first exchange.  PAIR: the norm of the row's other
-// component too; lines that keep one exponent (common) shift alike.
+// component too; lines loaded with one exponent (common) shift alike, unless
+// one of them has much more room than the other.
 template <int N, int E, bool WARP, bool PAIR> struct FxLine : LineSmem<FxC, E, WARP> {
   const uint32_t* l1;
   const uint32_t* l1_other;
@@ -74,11 +82,13 @@ template <int N, int E, bool WARP, bool PAIR> struct FxLine : LineSmem<FxC, E, W
       s += l1[w * stride];
       if (PAIR) t += l1_other[w * stride];
     }
-    if (PAIR && common) s = t = max(s, t);
     constexpr int kScaled = fx_transform_q<N, E, false>();
-    const int u = fx_room(s, kScaled - pre);
+    int u = fx_room(s, kScaled - pre);
+    if (PAIR) {
+      shift_other = fx_room(t, kScaled);
+      if (common && abs(u - shift_other) <= kFxUnlike) u = shift_other = min(u, shift_other);
+    }
     shift = u + pre;
-    if (PAIR) shift_other = fx_room(t, kScaled);
     return u;
   }
 };
@@ -443,7 +453,10 @@ struct FxRow {
   FxSplit m[2][2];   // phase of component i per |z_j|^2 (times 2^-twice)
   int sh[2];         // |z_j|^2 is shifted left by this before the product
   int twice;         // the phases come out times 2^-twice
-  int q[2];          // exponent of the components' lines in front of F_x
+  int qm[2];         // exponent of the components behind the matrix
+  int q[2];          // ... and of their lines in front of F_x
+  int dm[4];         // with the matrix of own exponents: shift of each product
+  bool split;        // take that one
   bool bad;
 };
 
@@ -470,17 +483,38 @@ __device__ __forceinline__ FxC fx_grow(FxSplit x, FxSplit y, FxC z, FxSplit w) {
   return FxC{fx_mul(x, w, z.x), fx_mul(y, w, z.y)};
 }
 
-// The interaction, matrix, interaction sequence in FP64, for a point whose
-// phases are too large for the series of fx_sincos / fx_expm1.  z comes with
-// exponents q and goes with exponents q + dq; m: the matrix, m01 and m10
-// unread (zero) without coupling.  (By value: an address would keep the points
-// of the common path in local memory.)
+// Components of unlike scale: the products of the matrix (tables of own
+// exponents e) meet at the exponent of the larger one, the other shifted down.
+// (Both are calls: their code in the common path costs its small passes, which
+// fetch their instructions anew in every launch, 3%.)
 struct FxPair {
   FxC z0, z1;
 };
-static __device__ __noinline__ FxPair fx_point_far(FxPair z, int q0, int q1, int dq, double lam2, double zr, double zi,
-                                                   double g_uu, double g_dd, double g_ud, double2 m00, double2 m01,
-                                                   double2 m10, double2 m11) {
+static __device__ __noinline__ void fx_split_exponents(FxRow* r, int q0, int q1, int4 e) {
+  const int t[4] = {q0 + 2 + e.x, q1 + 2 + e.y, q0 + 2 + e.z, q1 + 2 + e.w};
+  r->qm[0] = max(t[0], t[1]);
+  r->qm[1] = max(t[2], t[3]);
+  for (int k = 0; k < 4; ++k) r->dm[k] = min(63, r->qm[k / 2] - t[k]);
+}
+static __device__ __noinline__ FxPair fx_matrix_split(FxPair z, int4 m00, int4 m01, int4 m10, int4 m11,
+                                                      const int* dm) {
+  auto term = [](FxC z, int4 m, int d) {  // z m 2^(-64 - d), rounded
+    const FxC t = fx_cmul<false>(z, m);
+    const fx_t half = (fx_t(1) << d) >> 1;
+    return FxC{(t.x + half) >> d, (t.y + half) >> d};
+  };
+  return FxPair{cadd(term(z.z0, m00, dm[0]), term(z.z1, m01, dm[1])),
+                cadd(term(z.z0, m10, dm[2]), term(z.z1, m11, dm[3]))};
+}
+
+// The interaction, matrix, interaction sequence in FP64, for a point whose
+// phases are too large for the series of fx_sincos / fx_expm1.  z comes with
+// exponents q and goes with exponents qm; m: the matrix, m01 and m10
+// unread (zero) without coupling.  (By value: an address would keep the points
+// of the common path in local memory.)
+static __device__ __noinline__ FxPair fx_point_far(FxPair z, int q0, int q1, int qm0, int qm1, double lam2, double zr,
+                                                   double zi, double g_uu, double g_dd, double g_ud, double2 m00,
+                                                   double2 m01, double2 m10, double2 m11) {
   double2 p0 = make_double2(fx_to_double_far(z.z0.x, q0), fx_to_double_far(z.z0.y, q0));
   double2 p1 = make_double2(fx_to_double_far(z.z1.x, q1), fx_to_double_far(z.z1.y, q1));
   const double n0 = lam2 * cabs2(p0), n1 = lam2 * cabs2(p1);
@@ -490,8 +524,8 @@ static __device__ __noinline__ FxPair fx_point_far(FxPair z, int q0, int q1, int
   p1 = cmul(p1, i1);
   const double2 r0 = cmul(cadd(cmul(m00, p0), cmul(m01, p1)), i0);
   const double2 r1 = cmul(cadd(cmul(m11, p1), cmul(m10, p0)), i1);
-  return FxPair{FxC{__double2ll_rn(ldexp(r0.x, -(q0 + dq))), __double2ll_rn(ldexp(r0.y, -(q0 + dq)))},
-                FxC{__double2ll_rn(ldexp(r1.x, -(q1 + dq))), __double2ll_rn(ldexp(r1.y, -(q1 + dq)))}};
+  return FxPair{FxC{__double2ll_rn(ldexp(r0.x, -qm0)), __double2ll_rn(ldexp(r0.y, -qm0))},
+                FxC{__double2ll_rn(ldexp(r1.x, -qm1)), __double2ll_rn(ldexp(r1.y, -qm1))}};
 }
 
 template <int N, int E, int ROWS>
@@ -523,7 +557,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
 
   FxC v[1][E];
   int q, q_other;   // exponents of this line and of the row's other component
-  bool bad;
+  bool bad, common;
   {
     const int4* __restrict__ in = reinterpret_cast<const int4*>(a.in[comp]);
     int4 w[E];
@@ -563,9 +597,9 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
         other = max(other, s_mx[theirs + i]);
       }
     }
-    // components that a coupling mixes share one exponent
-    if (step && !a.op.diag) mx = other = max(mx, other);
-    const int be = fx_line_exp(mx), be_other = fx_line_exp(other);
+    int be = fx_line_exp(mx), be_other = fx_line_exp(other);
+    common = step && !a.op.diag && abs(be - be_other) <= kFxUnlike;
+    if (common) be = be_other = max(be, be_other);
     // a step's densities mix the components: one bad line spoils both
     bad = be == kFxNonFinite || (step && be_other == kFxNonFinite);
     q = fx_line_q(be, 62 - kBits);
@@ -589,7 +623,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   const int line = tid / T;
   FxC* const base = sm + (comp * ROWS + rho) * LS;
   const FxLine<N, E, kWarp, true> smv(base, WL, 1, s_l1 + line * WL, l1, s_l1 + (line ^ 1) * WL, l1_other,
-                                      step && !a.op.diag);
+                                      common);
   const FxC* tw = reinterpret_cast<const FxC*>(a.twf);
 
   if (step) {
@@ -618,7 +652,6 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
     if constexpr (kWarp) __syncthreads();  // the limbs of every warp
     q += kTq - smv.shift;
     q_other += kTq - smv.shift_other;
-    const int dq = 2 + a.me;  // the matrix tables are held as A 2^(62 - me)
     // the row's constants, by the first thread of each row
     if (comp == 0 && j == 0) {
       double w;
@@ -648,6 +681,11 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       r.pb = fx_factor(fx_from_words(xh, uint32_t(__double2loint(px)), be, 62),
                        fx_from_words(yh, uint32_t(__double2loint(py)), be, 62));
       const int qz[2] = {q, q_other};
+      // the matrix tables are held as A 2^(62 - e), the products scaled by 2^-64
+      r.qm[0] = q + 2 + a.me[0];
+      r.qm[1] = q_other + 2 + a.me[3];
+      r.split = !a.op.diag && (a.split || q != q_other);
+      if (r.split) fx_split_exponents(&r, q, q_other, make_int4(a.mse[0], a.mse[1], a.mse[2], a.mse[3]));
       const double ko = a.kz[2] * y2;
       const uint32_t oh = uint32_t(__double2hiint(ko));
       const uint32_t dh[2] = {uint32_t(__double2hiint(a.kz[0] * y2)), uint32_t(__double2hiint(a.kz[1] * y2))};
@@ -672,7 +710,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
         r.m[k][k] = fx_split((dh[k] << 1 | dl[k]) == 0 ? 0 : fx_from_words(dh[k], dl[k], bk, 62));
         r.m[1 - k][k] = fx_split(ko == 0.0 ? 0 : fx_from_words(oh, uint32_t(__double2loint(ko)), bk, 62));
         r.sh[k] = sh > 62 ? 63 : sh;  // past 62 every nonzero density goes the FP64 way
-        r.q[k] = qz[k] + dq + 64 + fx_line_q(be, 62) - h;
+        r.q[k] = r.qm[k] + 64 + fx_line_q(be, 62) - h;
       }
       r.bad = bad || be == kFxNonFinite || int(largest >> 20) == kFxNonFinite || whi < 0x100000 ||
               (whi >> 20) == kFxNonFinite;
@@ -703,7 +741,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       const FxSplit m00 = r.m[0][0], m01 = r.m[0][1], m10 = r.m[1][0], m11 = r.m[1][1];
       const int sh0 = r.sh[0], sh1 = r.sh[1], twice = r.twice;
       const fx_t lim0 = fx_t(1) << max(0, 62 - sh0), lim1 = fx_t(1) << max(0, 62 - sh1);
-      const bool diag = a.op.diag != 0, real = a.op.zi == 0.0;
+      const bool diag = a.op.diag != 0, split = r.split, real = a.op.zi == 0.0;
       const int q0 = comp == 0 ? q : q_other, q1 = comp == 0 ? q_other : q;
       // element x = jj + m 2T at padded position pad(jj) + m kStep when 2T is
       // a multiple of E (every power of two)
@@ -742,11 +780,18 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
             z1 = fx_turn(x1, y1, z1, w1);
           }
           x0 = fx_split(z0.x), y0 = fx_split(z0.y), x1 = fx_split(z1.x), y1 = fx_split(z1.y);
-          z0 = fx_cmul<false>(x0, y0, __ldg(a.mf[0] + x), FxC{0, 0});
-          z1 = fx_cmul<false>(x1, y1, __ldg(a.mf[3] + x), FxC{0, 0});
-          if (!diag) {
-            z0 = fx_cmul<false>(x1, y1, __ldg(a.mf[1] + x), z0);
-            z1 = fx_cmul<false>(x0, y0, __ldg(a.mf[2] + x), z1);
+          if (split) {
+            const FxPair u = fx_matrix_split(FxPair{z0, z1}, __ldg(a.ms[0] + x), __ldg(a.ms[1] + x),
+                                             __ldg(a.ms[2] + x), __ldg(a.ms[3] + x), r.dm);
+            z0 = u.z0;
+            z1 = u.z1;
+          } else {
+            z0 = fx_cmul<false>(x0, y0, __ldg(a.mf[0] + x), FxC{0, 0});
+            z1 = fx_cmul<false>(x1, y1, __ldg(a.mf[3] + x), FxC{0, 0});
+            if (!diag) {
+              z0 = fx_cmul<false>(x1, y1, __ldg(a.mf[1] + x), z0);
+              z1 = fx_cmul<false>(x0, y0, __ldg(a.mf[2] + x), z1);
+            }
           }
           x0 = fx_split(z0.x), y0 = fx_split(z0.y), x1 = fx_split(z1.x), y1 = fx_split(z1.y);
           if (real) {
@@ -759,7 +804,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
         } else {
           const double2 none = make_double2(0.0, 0.0);
           const FxPair far = fx_point_far(
-              FxPair{z0, z1}, q0, q1, dq, a.norm_num / s_w, a.op.zr, a.op.zi, a.g_uu, a.g_dd, a.g_ud, a.op.m[0].p[x],
+              FxPair{z0, z1}, q0, q1, r.qm[0], r.qm[1], a.norm_num / s_w, a.op.zr, a.op.zi, a.g_uu, a.g_dd, a.g_ud, a.op.m[0].p[x],
               diag ? none : a.op.m[1].p[x], diag ? none : a.op.m[2].p[x], a.op.m[3].p[x]);
           z0 = far.z0;
           z1 = far.z1;

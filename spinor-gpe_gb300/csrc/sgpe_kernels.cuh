@@ -216,8 +216,14 @@ enum RowMode { kRowStep = 0, kRowForward = 1, kRowInverse = 2 };
 template <typename R> struct RowFx {};
 template <> struct RowFx<double> {
   const int4* twf;       // twiddles of the x transform as split factors
-  const int4* mf[4];     // RealOp::m times 2^(62 - me)
-  int me;
+  // RealOp::m times 2^(62 - me), times 2^(62 - mse); with coupling the four of
+  // mf share one exponent and those of ms have their own (without: mf[0], mf[3]
+  // with their own)
+  const int4* mf[4];
+  int me[4];
+  const int4* ms[4];
+  int mse[4];
+  int split;             // the matrix leaves components of unlike scale: only ms will do
   double kz[3];          // (zi or zr) norm_num (g_uu, g_dd, g_ud)
   double sqrt_norm;      // sqrt(norm_num)
 };

@@ -177,6 +177,26 @@ def test_minority_component_keeps_its_precision(tp, tmp_path, amp):
         assert not got[1].any()
 
 
+# A component of 10^-k of the other's amplitude under a coupling, down to one
+# that the coupling alone fills, and a matrix whose rows differ (a detuning of
+# 500 damps one component by e^-10 in an imaginary step).  Each component's own
+# error: the FP64 oracle's is 1e-15 to 2e-15 of a component over three steps,
+# the bound five times that.
+@pytest.mark.parametrize('time,omega,delta', [
+    ('real', 1.0, 0.3), ('real', 1e-3, 0.3), ('real', 1e-6, 0.0), ('imag', 1e-3, 0.3), ('imag', 0.5, 500.0)])
+@pytest.mark.parametrize('amp', [(1.0, 1e-3), (1.0, 1e-6), (1e-6, 1.0), (1.0, 1e-9), (1.0, 0.0)])
+@pytest.mark.parametrize('nx,ny,n', [(64, 64, 1), (128, 64, 3), (512, 32, 3), (192, 384, 3), (2048, 32, 2)])
+def test_coupled_minority_component_keeps_its_precision(tp, tmp_path, nx, ny, n, amp, time, omega, delta):
+    ps = _problem(tmp_path, nx, ny, (1000.0, 995.0, 990.0), omega, delta=delta)
+    ps.psik = [p * a for p, a in zip(ps.psik, amp)]
+    dt = 1e-3 if time == 'real' else 0.02
+    ref, _ = _oracle(ps, dt, time, n)
+    prop = tp.TensorPropagator(ps, dt, n, 'cuda', time=time, dtype=128)
+    prop.full_steps(n)
+    for got, want in zip(prop.psik, ref):
+        assert rel_l2(got.cpu().numpy(), want) <= 1e-14
+
+
 def test_bad_state_stays_visible(tp, tmp_path):
     ps = _problem(tmp_path, 64, 64, (1000.0, 995.0, 990.0), 1.0)
     prop = tp.TensorPropagator(ps, 1e-3, 3, 'cuda', time='real', dtype=128)
