@@ -435,16 +435,40 @@ __device__ __forceinline__ void fx_limb_add(FxLimbs* s, double v, int be) {
   s->l[2] += (uint32_t(t & 0xffffu) << 8) | uint32_t(r >> 56);
 }
 // sum of the warps' limbs, times 2^q of one in the last of the 72 bits
-__device__ __forceinline__ double fx_limb_value(const FxLimbs* s, int stride, int warps, int be) {
+__device__ __forceinline__ double fx_limb_value(const FxLimbs* s, int warps, int be) {
   uint64_t a = 0, b = 0, c = 0;
   for (int w = 0; w < warps; ++w) {
-    a += s[w * stride].l[0];
-    b += s[w * stride].l[1];
-    c += s[w * stride].l[2];
+    a += s[w].l[0];
+    b += s[w].l[1];
+    c += s[w].l[2];
   }
   // the largest exponent's values lie in [2^71, 2^72) units
   const int q = be - 1023 - 71;
   return fx_to_double(fx_t((a << 24) + b), q + 24) + fx_to_double(fx_t(c), q);
+}
+
+// The populations from the column pass's partial sums [comp][tile][u, w] (or
+// their final sums), summed in FP64 by one warp of block 0 while the others wait
+// for the row's constants.  (A call, as above.)
+static __device__ __noinline__ void fx_populations(const double* part, const double* fin, int ntile, double atom_num,
+                                                   double* pops) {
+  const int lane = threadIdx.x & 31;
+  double u0 = 0.0, u1 = 0.0;
+  if (fin == nullptr) {
+    for (int i = lane; i < ntile; i += 32) {
+      u0 += part[2 * i];
+      u1 += part[2 * (ntile + i)];
+    }
+    u0 = warp_sum(u0);
+    u1 = warp_sum(u1);
+  } else {
+    u0 = fin[0];
+    u1 = fin[1];
+  }
+  if (lane == 0) {
+    pops[0] = atom_num * u0 / (u0 + u1);
+    pops[1] = atom_num * u1 / (u0 + u1);
+  }
 }
 
 // What the point-wise operators of one row share.
@@ -542,7 +566,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   __shared__ uint32_t s_l1[NT / 32], s_l1f[2 * ROWS], s_mxf[2 * ROWS];
   constexpr int NW = NT / 32;
   __shared__ uint32_t s_wmax[NW];
-  __shared__ FxLimbs s_limb[NW][3];  // sums of w, u_0, u_1 per warp
+  __shared__ FxLimbs s_limb[NW];     // sums of w per warp
   __shared__ FxRow s_row[ROWS];
   __shared__ double s_w;
 
@@ -553,7 +577,6 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
   const int y = pos.x * ROWS + rho;
   const long long row_off = (long long)y * N;
   const bool step = a.mode == kRowStep;
-  const bool want_u = a.pops != nullptr && pos.x == 0;
 
   FxC v[1][E];
   int q, q_other;   // exponents of this line and of the row's other component
@@ -568,10 +591,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
     if (step && a.fin == nullptr) {
       // the largest of the column pass's partial sums [comp][tile][u, w]
       uint32_t wm = 0;
-      for (int i = tid; i < 2 * a.ntile; i += NT) {
-        wm = max(wm, uint32_t(__double2hiint(a.part[2 * i + 1])));
-        if (want_u) wm = max(wm, uint32_t(__double2hiint(a.part[2 * i])));
-      }
+      for (int i = tid; i < 2 * a.ntile; i += NT) wm = max(wm, uint32_t(__double2hiint(a.part[2 * i + 1])));
       wm = __reduce_max_sync(0xffffffffu, wm);
       if ((tid & 31) == 0) s_wmax[tid >> 5] = wm;
     }
@@ -633,19 +653,12 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
 #pragma unroll
       for (int w = 0; w < NW; ++w) wm = max(wm, s_wmax[w]);
       bw = max(int(wm >> 20), 2);
-      auto warp_limbs = [&](int k, int i0, int i1, int part) {
-        FxLimbs s{};
-        for (int i = i0 + tid; i < i1; i += NT) fx_limb_add(&s, a.part[2 * i + part], bw);
+      FxLimbs s{};
+      for (int i = tid; i < 2 * a.ntile; i += NT) fx_limb_add(&s, a.part[2 * i + 1], bw);
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          const uint32_t x = __reduce_add_sync(0xffffffffu, s.l[l]);
-          if ((tid & 31) == 0) s_limb[tid >> 5][k].l[l] = x;
-        }
-      };
-      warp_limbs(0, 0, 2 * a.ntile, 1);
-      if (want_u) {
-        warp_limbs(1, 0, a.ntile, 0);
-        warp_limbs(2, a.ntile, 2 * a.ntile, 0);
+      for (int l = 0; l < 3; ++l) {
+        const uint32_t x = __reduce_add_sync(0xffffffffu, s.l[l]);
+        if ((tid & 31) == 0) s_limb[tid >> 5].l[l] = x;
       }
     }
     fft_lines<N, E, +1, 1, false, true>(v, j, smv, tw);
@@ -656,7 +669,7 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
     if (comp == 0 && j == 0) {
       double w;
       if (a.fin != nullptr) w = a.fin[2];
-      else w = bw >= kFxNonFinite ? __hiloint2double(kNanHi, 0) : fx_limb_value(&s_limb[0][0], 3, NW, bw);
+      else w = bw >= kFxNonFinite ? __hiloint2double(kNanHi, 0) : fx_limb_value(s_limb, NW, bw);
       // y = sqrt(1/w) 2^h by one third-order step from the FP32 root of w 2^-2h
       // in [1, 4) (FP64 operations are the longest chain of a small pass)
       const int whi = __double2hiint(w);
@@ -714,23 +727,9 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       }
       r.bad = bad || be == kFxNonFinite || int(largest >> 20) == kFxNonFinite || whi < 0x100000 ||
               (whi >> 20) == kFxNonFinite;
-      if (tid == 0) {
-        s_w = w;
-        if (want_u) {
-          double u0, u1;
-          if (a.fin != nullptr) {
-            u0 = a.fin[0];
-            u1 = a.fin[1];
-          } else {
-            const double nan = __hiloint2double(kNanHi, 0);
-            u0 = bw >= kFxNonFinite ? nan : fx_limb_value(&s_limb[0][1], 3, NW, bw);
-            u1 = bw >= kFxNonFinite ? nan : fx_limb_value(&s_limb[0][2], 3, NW, bw);
-          }
-          a.pops[0] = a.atom_num * u0 / (u0 + u1);
-          a.pops[1] = a.atom_num * u1 / (u0 + u1);
-        }
-      }
+      if (tid == 0) s_w = w;
     }
+    if (a.pops != nullptr && pos.x == 0 && tid >= NT - 32) fx_populations(a.part, a.fin, a.ntile, a.atom_num, a.pops);
     __syncthreads();
     {
       using LS0 = LineSmem<FxC, E>;

@@ -197,6 +197,22 @@ def test_coupled_minority_component_keeps_its_precision(tp, tmp_path, nx, ny, n,
         assert rel_l2(got.cpu().numpy(), want) <= 1e-14
 
 
+# populations of a minority: each to its own 1e-13 (they are sums of squares
+# that the oracle has to 1e-15)
+@pytest.mark.parametrize('amp', [1e-3, 1e-6, 1e-9])
+@pytest.mark.parametrize('omega', [None, 1e-4])
+@pytest.mark.parametrize('nx,ny', [(64, 64), (512, 128), (2048, 32)])
+def test_population_of_a_minority(tp, tmp_path, nx, ny, omega, amp):
+    ps = _problem(tmp_path, nx, ny, (1000.0, 995.0, 990.0), omega)
+    ps.psik = [ps.psik[0] * amp, ps.psik[1]]
+    _, ref = _oracle(ps, 1e-3, 'real', 4)
+    prop = tp.TensorPropagator(ps, 1e-3, 4, 'cuda', time='real', dtype=128)
+    pops = torch.empty((4, 2), dtype=torch.float64, device='cuda')
+    prop.full_steps(4, pops)
+    prop.psik
+    np.testing.assert_allclose(pops.cpu().numpy(), ref, rtol=1e-13)
+
+
 def test_bad_state_stays_visible(tp, tmp_path):
     ps = _problem(tmp_path, 64, 64, (1000.0, 995.0, 990.0), 1.0)
     prop = tp.TensorPropagator(ps, 1e-3, 3, 'cuda', time='real', dtype=128)
