@@ -426,8 +426,9 @@ struct FxLimbs {
 };
 __device__ __forceinline__ void fx_limb_add(FxLimbs* s, double v, int be) {
   const uint32_t hi = uint32_t(__double2hiint(v)), lo = uint32_t(__double2loint(v));
-  const uint64_t m = (uint64_t((hi << 11) | (lo >> 21) | 0x80000000u) << 32) | (lo << 11);
-  const int d = be - int(hi >> 20);        // below the largest exponent
+  const uint32_t e = hi >> 20;
+  const uint64_t m = (uint64_t((hi << 11) | (lo >> 21) | (e ? 0x80000000u : 0u)) << 32) | (lo << 11);
+  const int d = be - int(e ? e : 1);       // below the largest exponent (subnormals and zeros: exponent 1)
   const uint64_t t = fx_shr(m, d);         // the upper 64 bits
   const uint64_t r = d == 0 ? 0 : d < 64 ? m << (64 - d) : fx_shr(m, d - 64);
   s->l[0] += uint32_t(t >> 40);
@@ -672,9 +673,12 @@ __device__ __forceinline__ void row_body_fx(const RowArgs<double>& a, const Bloc
       else w = bw >= kFxNonFinite ? __hiloint2double(kNanHi, 0) : fx_limb_value(s_limb, NW, bw);
       // y = sqrt(1/w) 2^h by one third-order step from the FP32 root of w 2^-2h
       // in [1, 4) (FP64 operations are the longest chain of a small pass)
-      const int whi = __double2hiint(w);
-      const int h = ((whi >> 20) - 1023) >> 1;
-      const double wn = __hiloint2double(whi - (h << 21), __double2loint(w));
+      const bool tiny = __double2hiint(w) < 0x100000;
+      double ws = w;
+      if (tiny) ws *= 0x1p108;                   // out of the subnormal range
+      const int whi = __double2hiint(ws);        // still 0 when the norm is
+      const int hn = ((whi >> 20) - 1023) >> 1, h = tiny ? hn - 54 : hn;
+      const double wn = __hiloint2double(whi - (hn << 21), __double2loint(ws));
       const int wnh = __double2hiint(wn);
       const float y0 = rsqrtf(__int_as_float((((wnh >> 20) - 1023 + 127) << 23) | ((wnh & 0xfffff) << 3)));
       const int yb = __float_as_int(y0);

@@ -213,6 +213,30 @@ def test_population_of_a_minority(tp, tmp_path, nx, ny, omega, amp):
     np.testing.assert_allclose(pops.cpu().numpy(), ref, rtol=1e-13)
 
 
+# states without a norm: empty, or so small that every |psi|^2 underflows; and
+# one whose norm is subnormal, which still propagates like its multiple (the
+# subnormal sums carry 40 bits and more)
+@pytest.mark.parametrize('nx', [64, 512, 2048])
+@pytest.mark.parametrize('omega', [None, 1.0])
+def test_state_without_a_norm_stays_visible(tp, tmp_path, nx, omega):
+    ps = _problem(tmp_path, nx, 64, (1000.0, 995.0, 990.0), omega)
+    prop = tp.TensorPropagator(ps, 1e-3, 3, 'cuda', time='real', dtype=128)
+    psik = [p.clone() for p in prop.psik]
+    for scale in (0.0, 1e-200):
+        prop.psik = [p * scale for p in psik]
+        pops = torch.zeros((3, 2), dtype=torch.float64, device='cuda')
+        prop.full_steps(3, pops)
+        for p in prop.psik:
+            assert not torch.isfinite(torch.view_as_real(p)).any()
+        assert not torch.isfinite(pops).any()
+    got = []
+    for scale in (1.0, 1e-155):
+        prop.psik = [p * scale for p in psik]
+        prop.full_steps(3)
+        got.append(np.array([t.cpu().numpy() for t in prop.psik]))
+    assert rel_l2(got[1], got[0]) <= 1e-10
+
+
 def test_bad_state_stays_visible(tp, tmp_path):
     ps = _problem(tmp_path, 64, 64, (1000.0, 995.0, 990.0), 1.0)
     prop = tp.TensorPropagator(ps, 1e-3, 3, 'cuda', time='real', dtype=128)
