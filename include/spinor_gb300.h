@@ -125,9 +125,13 @@ int sgpe_single_step(sgpe_plan* plan, int sub, void* stream);
  * sgpe_store_psik with pops_dev = NULL, or the first sub-step of the next
  * sgpe_single_step / sgpe_full_steps), so pops_dev must stay valid until
  * then.  sgpe_load_psik discards that pending write.
- * Without populations, steady-state steps are replayed from CUDA graphs the
- * plan captures on first use (one graph launch per 8 steps); changing the
- * physics or operators discards them.
+ * Steady-state steps are replayed from CUDA graphs the plan captures on first
+ * use (one graph launch per 8 steps); changing the physics or operators
+ * discards them.  With populations the graphs are captured when the plan has
+ * taken 128 such steps (at once for double-float plans and complex128 plans of
+ * 512 x 256 points and more) and are followed by a copy of the populations to
+ * pops_dev; while `stream` is being captured by the caller, steps with
+ * populations are launched one by one, so that the capture holds them.
  * Replaces: TensorPropagator.full_step (tensor_propagator.py:214-222) and the
  * step loop of prop_loop (:185-194). */
 int sgpe_full_steps(sgpe_plan* plan, int n_steps, double* pops_dev, void* stream);

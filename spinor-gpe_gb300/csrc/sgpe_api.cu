@@ -210,7 +210,8 @@ struct sgpe_plan {
   // the same steps writing the populations in front of each step to pops_buf
   // (kGraphSteps pairs); a launch is followed by a copy to the caller's rows
   cudaGraphExec_t graph_pops[2] = {nullptr, nullptr};
-  double* pops_buf = nullptr;
+  double* pops_buf = nullptr;   // behind `derr`, in its allocation
+  int pops_steps = 0;           // steps with populations since the graphs were dropped, up to kPopsSteps
   bool graphs_enabled = true;
   // incremented whenever captured launches would go stale (new physics or
   // operators); batches compare it with the value at their capture
@@ -219,6 +220,7 @@ struct sgpe_plan {
 
 namespace {
 constexpr int kGraphSteps = 8;
+constexpr int kPopsSteps = 128;
 }
 
 // A set of plans stepped together: their steady-state steps are captured as
@@ -1297,6 +1299,7 @@ template <typename R> void update_col_tmaps(sgpe_plan* p) {
 
 void drop_graphs(sgpe_plan* p) {
   ++p->epoch;
+  p->pops_steps = 0;
   for (auto* set : {&p->graph, &p->graph_pops})
     for (auto& g : *set) {
       if (g) cudaGraphExecDestroy(g);
@@ -1399,9 +1402,16 @@ int apply_shapes_any(sgpe_plan* p, int rs, int cs) {
 // Steady-state steps are replayed from graphs.  With populations, the step
 // that follows another writes the populations of the state between them: a
 // graph's steps write them to the plan's buffer, copied to the caller's rows
-// behind each launch (launched one by one, the six passes of a 512^2
-// complex64 step took 40.6 us of host time against 36 us on the GPU, and
-// 70 us against 53 us at 256 x 128 complex128).
+// behind each launch.  Their two graphs take 0.3 ms to make, in the call of a
+// user that often makes only one.  Steps that are long against their launches
+// (40 us of host time; every double-float step, complex128 from 512 x 256 on)
+// gain from a graph at once, and its capture hides behind two steps launched
+// first, serially as in the graph (overlapped they take up to 1.8 times as
+// long, overlap_launches).  The others gain 0.2-4 us a step, and their graphs
+// are made when the plan has taken kPopsSteps such steps.  us of a new plan's
+// first 40 steps, graphs at once / so: complex64 64^2 1,179 / 905, 512^2 2,005 /
+// 1,810, complex128 256 x 128 2,554 / 2,226, 512^2 5,801 / 5,945, double-float
+// 256^2 4,743 / 4,726; repeated, complex64 512^2 1,549 / 1,545.
 template <typename R> int full_steps_impl(sgpe_plan* p, int n_steps, double* pops, cudaStream_t s) {
   // a caller that captures the stream itself gets the launches of its steps
   bool eager_pops = !p->graphs_enabled;
@@ -1410,20 +1420,22 @@ template <typename R> int full_steps_impl(sgpe_plan* p, int n_steps, double* pop
     const cudaError_t e = cudaStreamIsCapturing(s, &st);
     if (e != cudaSuccess) return cuda_fail(e, "capture status");
     eager_pops = st != cudaStreamCaptureStatusNone;
-    if (!eager_pops && p->pops_buf == nullptr &&
-        cudaMalloc(reinterpret_cast<void**>(&p->pops_buf), 2 * kGraphSteps * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      p->pops_buf = nullptr;
-      eager_pops = true;
-    }
+    // the tables of a step behind a step, which a capture could not make (steps
+    // with populations apply its two kinetic halves one after the other)
+    const int rc = eager_pops || !p->graphs_enabled ? SGPE_OK : ensure_pair(p, 0, 0);
+    if (rc != SGPE_OK) return rc;
   }
+  const bool long_step =
+      std::is_same<R, sgpe::DF>::value || (std::is_same<R, double>::value && (long long)p->nx * p->ny >= 512 * 256);
   int i = 0;
   while (i < n_steps) {
     double* slot = (pops != nullptr && i > 0) ? pops + 2 * (i - 1) : nullptr;
-    const bool steady = p->graphs_enabled && p->pending_pops == nullptr && p->form == kMixed && p->prev_sub == 0 &&
-                        (pops == nullptr || (i > 0 && !eager_pops));
+    const int k = (n_steps - i >= kGraphSteps) ? 1 : 0;
+    bool steady = p->graphs_enabled && p->pending_pops == nullptr && p->form == kMixed && p->prev_sub == 0;
+    if (steady && pops != nullptr)
+      steady = i > 0 && !eager_pops && (p->pops_steps >= kPopsSteps || (long_step && k == 1 && i >= 2));
     if (steady) {
-      const int k = (n_steps - i >= kGraphSteps) ? 1 : 0, steps = k ? kGraphSteps : 1;
+      const int steps = k ? kGraphSteps : 1;
       cudaGraphExec_t& g = (slot != nullptr ? p->graph_pops : p->graph)[k];
       if (g == nullptr) {
         const int rc = capture_steps<R>(p, steps, slot != nullptr ? p->pops_buf : nullptr, &g);
@@ -1431,13 +1443,17 @@ template <typename R> int full_steps_impl(sgpe_plan* p, int n_steps, double* pop
       }
       cudaError_t e = cudaGraphLaunch(g, s);
       if (e == cudaSuccess && slot != nullptr)
-        e = cudaMemcpyAsync(slot, p->pops_buf, 2 * steps * sizeof(double), cudaMemcpyDeviceToDevice, s);
+        e = cudaMemcpyAsync(slot, p->pops_buf, 2 * steps * sizeof(double), cudaMemcpyDefault, s);
       if (e != cudaSuccess) return cuda_fail(e, "graph launch");
+      if (pops != nullptr) p->pops_steps = std::min(p->pops_steps + steps, kPopsSteps);
       i += steps;
       continue;
     }
+    p->serial = pops != nullptr && long_step;
     const int rc = eager_step<R>(p, slot, s);
+    p->serial = false;
     if (rc != SGPE_OK) return rc;
+    if (pops != nullptr && p->pops_steps < kPopsSteps) ++p->pops_steps;
     ++i;
   }
   return SGPE_OK;
@@ -1509,8 +1525,14 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
       (upload_twiddles_fx(nx, sgpe::row_points_per_thread<double>(nx, p->row_shape), &p->twf_x) != SGPE_OK ||
        upload_twiddles_fx(ny, sgpe::col_points_per_thread<double>(ny, p->col_shape), &p->twf_y) != SGPE_OK))
     e = cudaErrorMemoryAllocation;
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->derr), sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(p->derr, 0, sizeof(int));
+  // the error word, and the populations that graphs write
+  const size_t pops_at = 16;
+  if (e == cudaSuccess)
+    e = cudaMalloc(reinterpret_cast<void**>(&p->derr), pops_at + 2 * kGraphSteps * sizeof(double));
+  if (e == cudaSuccess) {
+    p->pops_buf = reinterpret_cast<double*>(reinterpret_cast<char*>(p->derr) + pops_at);
+    e = cudaMemset(p->derr, 0, sizeof(int));
+  }
   if (e != cudaSuccess) {
     sgpe_plan_destroy(p);
     return fail(SGPE_ERR_OOM, std::string("plan allocation: ") + cudaGetErrorString(e));
@@ -1547,7 +1569,6 @@ int sgpe_plan_destroy(sgpe_plan* p) {
     if (p->epsi[c]) cudaFree(p->epsi[c]);
   if (p->epart) cudaFree(p->epart);
   if (p->tcb) cudaFree(p->tcb);
-  if (p->pops_buf) cudaFree(p->pops_buf);
   if (p->apart) cudaFree(p->apart);
   if (p->tmaps) cudaFree(p->tmaps);
   if (p->derr) cudaFree(p->derr);

@@ -246,3 +246,46 @@ def test_bad_state_stays_visible(tp, tmp_path):
     prop.full_steps(3)
     for p in prop.psik:
         assert not torch.isfinite(torch.view_as_real(p)).any()
+
+
+# steps with populations: eager ones, the graphs of long steps (made within the
+# first call) and those made after 128 steps all give the same bits
+@pytest.mark.parametrize('dtype', [64, 128, 'double-float'])
+@pytest.mark.parametrize('nx,ny', [(64, 64), (512, 256)])
+def test_population_graphs_match_eager_steps(tp, tmp_path, monkeypatch, dtype, nx, ny):
+    ps = _problem(tmp_path, nx, ny, (1000.0, 995.0, 990.0), 1.0)
+    props = [tp.TensorPropagator(ps, 1e-3, 20, 'cuda', time='real', dtype=dtype)]
+    monkeypatch.setenv('SGPE_DISABLE_GRAPHS', '1')
+    props.append(tp.TensorPropagator(ps, 1e-3, 20, 'cuda', time='real', dtype=dtype))
+    for n in (20, 2, 110, 9, 21):
+        out = []
+        for p in props:
+            pops = torch.full((n, 2), -1.0, dtype=torch.float64, device='cuda')
+            p.full_steps(n, pops)
+            out.append([t.cpu().numpy() for t in p.psik] + [pops.cpu().numpy()])
+        for a, b in zip(*out):
+            np.testing.assert_array_equal(a, b)
+
+
+# a stream that the caller captures gets the launches of the steps
+@pytest.mark.parametrize('nx,ny', [(64, 64), (512, 256)])
+def test_populations_on_a_captured_stream(tp, tmp_path, nx, ny):
+    ps = _problem(tmp_path, nx, ny, (1000.0, 995.0, 990.0), 1.0)
+    a, b = (tp.TensorPropagator(ps, 1e-3, 20, 'cuda', time='real', dtype=128) for _ in range(2))
+    out = []
+    for p in (a, b):
+        pops = torch.zeros((12, 2), dtype=torch.float64, device='cuda')
+        p.full_steps(12, pops)     # makes the merged tables
+        p.full_steps(1)
+        pops.zero_()
+        if p is a:
+            p.full_steps(12, pops)
+        else:
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                p.full_steps(12, pops)
+            graph.replay()
+        out.append([t.cpu().numpy() for t in p.psik] + [pops.cpu().numpy()])
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
