@@ -62,7 +62,6 @@ struct HostField {
 struct SepOps {
   DevField kx[2], ky[2];
   bool kin = false, kin_real = false;
-  DevField px[2], py[2], s01x, s10x;
   bool pot = false, cpl = false;
   // The real-space operators of the separable row kernels, one 2x2 matrix
   // per point: coupling, potential and coupling C P C = pb(y) A(x) with
@@ -75,10 +74,10 @@ struct SepOps {
   // complex128 plans: the same tables as split fixed-point factors
   // (sgpe_fx.cuh), times 2^-exponent; not made when a table holds a value
   // that is not finite
-  void* fky[2] = {nullptr, nullptr};
-  void* fm = nullptr;    // m[0..3] one after the other, with one exponent
-  void* fms = nullptr;   // ... with an exponent each
-  void* fdg = nullptr;   // dg[0..1]
+  const int4* fky[2] = {nullptr, nullptr};
+  const int4* fm = nullptr;    // m[0..3] one after the other, with one exponent
+  const int4* fms = nullptr;   // ... with an exponent each
+  const int4* fdg = nullptr;   // dg[0..1]
   int fke[2] = {0, 0}, fme = 0, fmse[4] = {0, 0, 0, 0}, fdge[2] = {0, 0};
   bool fx_kin = false, fx_c = false, fx_d = false;
 };
@@ -177,9 +176,9 @@ struct sgpe_plan {
   uint32_t* tcb = nullptr;   // their B fragments (device)
   void* tw_x = nullptr;
   void* tw_y = nullptr;
-  // twiddles of the fixed-point passes (complex128 plans)
-  void* twf_x = nullptr;
-  void* twf_y = nullptr;
+  // twiddles of the fixed-point passes (complex128 plans), behind tw_x, tw_y
+  const int4* twf_x = nullptr;
+  const int4* twf_y = nullptr;
   // complex128 twiddle tables of a double-float plan, for its complex128
   // transforms (sgpe_fft2, the energy functional); made on first use
   void* tw64_x = nullptr;
@@ -293,11 +292,67 @@ template <class F> auto by_iface(int bits, F&& f) {
   return f(double{});
 }
 
+// Split fixed-point factor (fx_cmul) of two 64-bit integers.
+int4 fx_entry(long long re, long long im) {
+  auto split = [](long long w, int* h, int* l) {
+    *l = int(uint32_t(uint64_t(w)));
+    if (*l == INT32_MIN) ++*l;  // the kernels negate low words
+    *h = int((w - *l) >> 32);
+  };
+  int4 r;
+  split(re, &r.x, &r.y);
+  split(im, &r.z, &r.w);
+  return r;
+}
+
+// Twiddle table of an (n, e) transform in fixed point: the entries of
+// upload_twiddles times 2^(64 - fx_bits) (sgpe_fx.cuh).  The roots of
+// order n are products of two short tables evaluated in extended precision,
+// rounded at 2^-62 (evaluating every root so took 2 ms a plan).
+std::vector<int4> twiddles_fx(int n, int e) {
+  struct Root {
+    long long re, im;  // times 2^62
+  };
+  // of order sqrt(n): the fewest roots in extended precision (setting up a
+  // 256^2 solve took 4.25 ms with 64 fine roots, under 3.95 with 16)
+  int kFine = 8;
+  while (kFine * kFine < n) kFine *= 2;
+  const long double two_pi = 6.283185307179586476925286766559005768L;
+  auto root = [&](int m) {
+    long double sn, cs;
+    sincosl(two_pi * (long double)m / (long double)n, &sn, &cs);
+    return Root{llrintl(cs * 0x1p62L), llrintl(-sn * 0x1p62L)};
+  };
+  std::vector<Root> fine(kFine), coarse((n + kFine - 1) / kFine);
+  for (int m = 0; m < kFine; ++m) fine[m] = root(m);
+  for (size_t m = 0; m < coarse.size(); ++m) coarse[m] = root(int(m) * kFine);
+  auto scaled = [](__int128 v, int bits) { return (long long)((v + ((__int128)1 << (bits - 1))) >> bits); };
+  std::vector<int4> h;
+  h.reserve(sgpe::tw_offset(n, e, n));
+  for (int ns = 1; ns < n;) {
+    const int rs = sgpe::stage_radix(n, e, ns);
+    const int len = ns * rs;
+    const int down = 60 + sgpe::fx_bits(rs);  // 2^124 -> 2^(64 - bits)
+    for (int r = 1; r < rs; ++r)
+      for (int k = 0; k < ns; ++k) {
+        const int m = int(((long long)k * r) % len) * (n / len);
+        const Root &a = fine[m % kFine], &b = coarse[m / kFine];
+        const __int128 re = (__int128)a.re * b.re - (__int128)a.im * b.im;
+        const __int128 im = (__int128)a.re * b.im + (__int128)a.im * b.re;
+        h.push_back(fx_entry(scaled(re, down), scaled(im, down)));
+      }
+    ns = len;
+  }
+  return h;
+}
+
 // Per-stage twiddle table of an (n, e) transform, in the order the FFT
 // engine reads it (sgpe_fft.cuh: tw_offset): for each stage (ns, r_s),
 // entries exp(-2 pi i k r / (ns r_s)) at (r - 1) * ns + k.  Angles are
 // reduced exactly in integers and evaluated in FP64, then rounded once.
-template <typename R> void* upload_twiddles(int n, int e, cudaError_t* err) {
+// fx non-null (complex128): the fixed-point table follows in the same
+// allocation, at *fx.
+template <typename R> void* upload_twiddles(int n, int e, cudaError_t* err, const int4** fx = nullptr) {
   using W = sgpe::TwE<R>;
   std::vector<W> h;
   const double two_pi = 6.283185307179586476925286766559;
@@ -313,72 +368,21 @@ template <typename R> void* upload_twiddles(int n, int e, cudaError_t* err) {
     ns *= rs;
   }
   if (h.empty()) h.push_back(twiddle_entry<W>(1.0, 0.0));
+  const size_t n_own = h.size();
+  if constexpr (std::is_same<R, double>::value) {
+    if (fx != nullptr) {
+      static_assert(sizeof(W) == sizeof(int4), "one table behind the other");
+      const std::vector<int4> f = twiddles_fx(n, e);
+      h.resize(n_own + f.size());
+      std::memcpy(static_cast<void*>(h.data() + n_own), f.data(), sizeof(int4) * f.size());
+    }
+  }
   void* d = nullptr;
   *err = cudaMalloc(&d, sizeof(W) * h.size());
   if (*err != cudaSuccess) return nullptr;
   *err = cudaMemcpy(d, h.data(), sizeof(W) * h.size(), cudaMemcpyHostToDevice);
+  if (fx != nullptr) *fx = reinterpret_cast<const int4*>(static_cast<const W*>(d) + n_own);
   return d;
-}
-
-// Split fixed-point factor (fx_cmul) of two 64-bit integers.
-int4 fx_entry(long long re, long long im) {
-  auto split = [](long long w, int* h, int* l) {
-    *l = int(uint32_t(uint64_t(w)));
-    if (*l == INT32_MIN) ++*l;  // the kernels negate low words
-    *h = int((w - *l) >> 32);
-  };
-  int4 r;
-  split(re, &r.x, &r.y);
-  split(im, &r.z, &r.w);
-  return r;
-}
-
-int upload_int4(const std::vector<int4>& h, void** out, std::vector<void*>* allocs, const char* name) {
-  cudaError_t e = cudaMalloc(out, sizeof(int4) * h.size());
-  if (e != cudaSuccess) return fail(SGPE_ERR_OOM, std::string(name) + ": " + cudaGetErrorString(e));
-  if (allocs != nullptr) allocs->push_back(*out);
-  e = cudaMemcpy(*out, h.data(), sizeof(int4) * h.size(), cudaMemcpyHostToDevice);
-  return e == cudaSuccess ? SGPE_OK : cuda_fail(e, name);
-}
-
-// Twiddle table of an (n, e) transform in fixed point: the entries of
-// upload_twiddles times 2^(64 - fx_bits) (sgpe_fx.cuh).  The roots of
-// order n are products of two short tables evaluated in extended precision,
-// rounded at 2^-62 (evaluating every root so took 2 ms a plan).
-int upload_twiddles_fx(int n, int e, void** out) {
-  struct Root {
-    long long re, im;  // times 2^62
-  };
-  // of order sqrt(n): the fewest roots in extended precision (setting up a
-  // 256^2 solve took 4.25 ms with 64 fine roots, under 3.95 with 16)
-  int kFine = 8;
-  while (kFine * kFine < n) kFine *= 2;
-  const long double two_pi = 6.283185307179586476925286766559005768L;
-  auto root = [&](int m) {
-    const long double a = two_pi * (long double)m / (long double)n;
-    return Root{llrintl(ldexpl(cosl(a), 62)), llrintl(ldexpl(-sinl(a), 62))};
-  };
-  std::vector<Root> fine(kFine), coarse((n + kFine - 1) / kFine);
-  for (int m = 0; m < kFine; ++m) fine[m] = root(m);
-  for (size_t m = 0; m < coarse.size(); ++m) coarse[m] = root(int(m) * kFine);
-  auto scaled = [](__int128 v, int bits) { return (long long)((v + ((__int128)1 << (bits - 1))) >> bits); };
-  std::vector<int4> h;
-  for (int ns = 1; ns < n;) {
-    const int rs = sgpe::stage_radix(n, e, ns);
-    const int len = ns * rs;
-    const int down = 60 + sgpe::fx_bits(rs);  // 2^124 -> 2^(64 - bits)
-    for (int r = 1; r < rs; ++r)
-      for (int k = 0; k < ns; ++k) {
-        const int m = int(((long long)k * r) % len) * (n / len);
-        const Root &a = fine[m % kFine], &b = coarse[m / kFine];
-        const __int128 re = (__int128)a.re * b.re - (__int128)a.im * b.im;
-        const __int128 im = (__int128)a.re * b.im + (__int128)a.im * b.re;
-        h.push_back(fx_entry(scaled(re, down), scaled(im, down)));
-      }
-    ns = len;
-  }
-  if (h.empty()) h.push_back(fx_entry(1ll << 62, 0));
-  return upload_int4(h, out, nullptr, "fixed-point twiddles");
 }
 
 // Default kernel shape of a pass (axis 0: rows along x, 1: columns along y)
@@ -567,36 +571,76 @@ HostField host_field(const sgpe_field& f) {
 // Exponent of a table of zeros: below any sum it can be a term of.
 constexpr int kFxZeroTable = -4096;
 
+// Products with 2^e, in two factors (either alone is in the exponent range).
+struct PowerOfTwo {
+  double a, b;
+  explicit PowerOfTwo(int e) : a(std::ldexp(1.0, e / 2)), b(std::ldexp(1.0, e - e / 2)) {}
+  double operator*(double v) const { return v * a * b; }
+};
+
 // Smallest e with every |value| of the fields at most 2^e (to rounding);
 // false when a value is not finite.
 bool fx_exponent(std::initializer_list<const HostField*> fields, int* e) {
+  double part = 0.0, bad = 0.0;
+  for (const HostField* f : fields)
+    for (const double v : f->v) {
+      part = std::max(part, std::fabs(v));
+      bad += v * 0.0;   // NaN from an infinity or a NaN
+    }
+  if (!(bad == 0.0)) return false;
+  *e = kFxZeroTable;
+  if (part == 0.0) return true;
+  // |value|^2 over the largest part's power of two, in (1/4, 2]
+  int ep = 0;
+  std::frexp(part, &ep);
+  const PowerOfTwo unit(-ep);
   double most = 0.0;
   for (const HostField* f : fields)
     for (size_t i = 0; i < f->v.size(); i += 2) {
-      const double m = std::hypot(f->v[i], f->v[i + 1]);
-      if (!std::isfinite(m)) return false;
-      most = std::max(most, m);
+      const double x = unit * f->v[i], y = unit * f->v[i + 1];
+      most = std::max(most, x * x + y * y);
     }
-  *e = kFxZeroTable;
-  if (most > 0.0) std::frexp(most * (1.0 - 1e-9), e);
+  std::frexp(std::sqrt(most) * (1.0 - 1e-9), e);
+  *e += ep;
   return true;
 }
 
-// Tables of equal length as split fixed-point factors, value 2^(62 - e) (e of
-// each table), one after the other.
-int upload_fx(std::initializer_list<const HostField*> fields, const int* e, void** out, std::vector<void*>* allocs) {
+// Fixed-point tables gathered on the host and uploaded in one piece: split
+// factors of value 2^(62 - e) (e of each table).
+struct FxTables {
   std::vector<int4> h;
-  for (const HostField* f : fields) {
-    for (size_t i = 0; i < f->v.size(); i += 2)
-      h.push_back(fx_entry(std::llrint(std::ldexp(f->v[i], 62 - *e)), std::llrint(std::ldexp(f->v[i + 1], 62 - *e))));
-    ++e;
+  std::vector<std::pair<const int4**, size_t>> out;
+  // tables one behind the other, *p to point to the first
+  void add(std::initializer_list<const HostField*> fields, const int* e, const int4** p) {
+    out.push_back({p, h.size()});
+    for (const HostField* f : fields) {
+      const PowerOfTwo unit(*e == kFxZeroTable ? 0 : 62 - *e);
+      ++e;
+      for (size_t i = 0; i < f->v.size(); i += 2) h.push_back(fx_entry(integer(unit * f->v[i]), integer(unit * f->v[i + 1])));
+    }
   }
-  return upload_int4(h, out, allocs, "fixed-point table");
-}
+  int upload(std::vector<void*>* allocs) {
+    if (h.empty()) return SGPE_OK;
+    void* d = nullptr;
+    cudaError_t e = cudaMalloc(&d, sizeof(int4) * h.size());
+    if (e != cudaSuccess) return fail(SGPE_ERR_OOM, std::string("fixed-point tables: ") + cudaGetErrorString(e));
+    allocs->push_back(d);
+    e = cudaMemcpy(d, h.data(), sizeof(int4) * h.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_fail(e, "fixed-point tables");
+    for (const auto& o : out) *o.first = static_cast<const int4*>(d) + o.second;
+    return SGPE_OK;
+  }
+  // nearest integer (|v| < 2^62.1)
+  static long long integer(double v) {
+    const long long t = (long long)v;
+    const double r = v - double(t);
+    return t + (r >= 0.5) - (r <= -0.5);
+  }
+};
 
 // Kinetic part of SepOps from the FP64 factors of each component.
 int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2], SepOps* so,
-                  std::vector<void*>* allocs) {
+                  std::vector<void*>* allocs, FxTables* fx) {
   HostField x[2], y[2];
   for (int c = 0; c < 2; ++c)
     if (!split_xy(a[c], b[c], p->nx, p->ny, &x[c], &y[c])) return SGPE_OK;  // not separable: generic path
@@ -607,12 +651,10 @@ int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2]
   }
   so->kin = true;
   if (p->bits != 128) return SGPE_OK;
-  for (int c = 0; c < 2; ++c) {
-    int ex = 0;
+  int ex = 0;
+  for (int c = 0; c < 2; ++c)
     if (!fx_exponent({&x[c]}, &ex) || !fx_exponent({&y[c]}, &so->fke[c])) return SGPE_OK;
-    const int rc = upload_fx({&y[c]}, &so->fke[c], &so->fky[c], allocs);
-    if (rc != SGPE_OK) return rc;
-  }
+  for (int c = 0; c < 2; ++c) fx->add({&y[c]}, &so->fke[c], &so->fky[c]);
   so->fx_kin = true;
   return SGPE_OK;
 }
@@ -628,7 +670,7 @@ int build_sep_kin(sgpe_plan* p, const HostField (&a)[2], const HostField (&b)[2]
 // d0 = pa_0(x), d1 = kappa pa_1(x), all in FP64.  Leaves both fused flags
 // false when the y factors are not proportional.
 int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2], const HostField* s01,
-                const HostField* s10, double cr, double ci, SepOps* so, std::vector<void*>* allocs) {
+                const HostField* s10, double cr, double ci, SepOps* so, std::vector<void*>* allocs, FxTables* fxt) {
   typedef std::complex<double> cd;
   const int nx = p->nx, ny = p->ny;
   auto at = [](const HostField& f, int i) { return cd(f.v[2 * i], f.v[2 * i + 1]); };
@@ -671,8 +713,7 @@ int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2]
   so->fused_d = true;
   const bool fx = p->bits == 128;
   if (fx && fx_exponent({&dg[0]}, &so->fdge[0]) && fx_exponent({&dg[1]}, &so->fdge[1])) {
-    rc = upload_fx({&dg[0], &dg[1]}, so->fdge, &so->fdg, allocs);
-    if (rc != SGPE_OK) return rc;
+    fxt->add({&dg[0], &dg[1]}, so->fdge, &so->fdg);
     so->fx_d = true;
   }
   if (s01 != nullptr) {
@@ -682,9 +723,8 @@ int build_fused(sgpe_plan* p, const HostField (&px)[2], const HostField (&py)[2]
     if (fx && fx_exponent({&m[0], &m[1], &m[2], &m[3]}, &so->fme)) {
       for (int k = 0; k < 4; ++k) fx_exponent({&m[k]}, &so->fmse[k]);
       const int one[4] = {so->fme, so->fme, so->fme, so->fme};
-      rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, one, &so->fm, allocs);
-      if (rc == SGPE_OK) rc = upload_fx({&m[0], &m[1], &m[2], &m[3]}, so->fmse, &so->fms, allocs);
-      if (rc != SGPE_OK) return rc;
+      fxt->add({&m[0], &m[1], &m[2], &m[3]}, one, &so->fm);
+      fxt->add({&m[0], &m[1], &m[2], &m[3]}, so->fmse, &so->fms);
       so->fx_c = true;
     }
   }
@@ -733,14 +773,14 @@ int ensure_pair(sgpe_plan* p, int prev, int next) {
   for (int c = 0; c < 2; ++c) {
     ma[c] = multiply_fields(p->sub[prev].kin_host[c][0], p->sub[next].kin_host[c][0], p->nx, p->ny);
     mb[c] = multiply_fields(p->sub[prev].kin_host[c][1], p->sub[next].kin_host[c][1], p->nx, p->ny);
-    int rc = upload_host_field(p, ma[c], &po.a[c], &po.allocs);
-    if (rc == SGPE_OK) rc = upload_host_field(p, mb[c], &po.b[c], &po.allocs);
-    if (rc != SGPE_OK) {
-      free_pair(po);
-      return rc;
-    }
   }
-  const int rc = build_sep_kin(p, ma, mb, &po.sep, &po.allocs);
+  FxTables fx;
+  int rc = build_sep_kin(p, ma, mb, &po.sep, &po.allocs, &fx);
+  for (int c = 0; c < 2 && rc == SGPE_OK && !po.sep.kin; ++c) {
+    rc = upload_host_field(p, ma[c], &po.a[c], &po.allocs);
+    if (rc == SGPE_OK) rc = upload_host_field(p, mb[c], &po.b[c], &po.allocs);
+  }
+  if (rc == SGPE_OK) rc = fx.upload(&po.allocs);
   if (rc != SGPE_OK) {
     free_pair(po);
     return rc;
@@ -836,12 +876,12 @@ void col_fx<double>(const sgpe_plan* p, std::initializer_list<const SepOps*> ops
   for (const SepOps* s : ops) {
     if (!s->fx_kin) return;
     for (int c = 0; c < 2; ++c) {
-      a->kb[i][c] = static_cast<const int4*>(s->fky[c]);
+      a->kb[i][c] = s->fky[c];
       a->ke[i][c] = s->fke[c];
     }
     ++i;
   }
-  a->twf = static_cast<const int4*>(p->twf_y);
+  a->twf = p->twf_y;
 }
 
 // Whether the row pass of sub-step `so` can run in fixed point: separable
@@ -857,18 +897,18 @@ bool row_fx_ok(const sgpe_plan* p, const SubOps& so) {
 template <typename R> void row_fx(const sgpe_plan*, const SubOps&, sgpe::RowArgs<R>*) {}
 template <> void row_fx<double>(const sgpe_plan* p, const SubOps& so, sgpe::RowArgs<double>* a) {
   if (!row_fx_ok(p, so)) return;
-  const int4* m = static_cast<const int4*>(p->coupling ? so.sep.fm : so.sep.fdg);
+  const int4* m = p->coupling ? so.sep.fm : so.sep.fdg;
   for (int k = 0; k < 4; ++k) {
     a->mf[k] = m + (p->coupling ? k : k / 2) * p->nx;
     a->me[k] = p->coupling ? so.sep.fme : so.sep.fdge[k / 2];
-    a->ms[k] = p->coupling ? static_cast<const int4*>(so.sep.fms) + k * p->nx : nullptr;
+    a->ms[k] = p->coupling ? so.sep.fms + k * p->nx : nullptr;
     a->mse[k] = so.sep.fmse[k];
   }
   a->split = std::abs(std::max(a->mse[0], a->mse[1]) - std::max(a->mse[2], a->mse[3])) > sgpe::kFxUnlike;
   const double z = (so.zi != 0.0 ? so.zi : so.zr) * a->norm_num;
   for (int k = 0; k < 3; ++k) a->kz[k] = z * p->g[k];
   a->sqrt_norm = std::sqrt(a->norm_num);
-  a->twf = static_cast<const int4*>(p->twf_x);
+  a->twf = p->twf_x;
 }
 
 // Column pass over the state (in place) ending a sub-step and starting `sub`.
@@ -1168,8 +1208,8 @@ template <typename R> int fft2(sgpe_plan* p, const void* i0, const void* i1, voi
   c.scale = R(1);
   if constexpr (std::is_same<R, double>::value) {
     if (own) {
-      r.twf = static_cast<const int4*>(p->twf_x);
-      c.twf = static_cast<const int4*>(p->twf_y);
+      r.twf = p->twf_x;
+      c.twf = p->twf_y;
     }
   }
   cudaError_t e;
@@ -1363,30 +1403,29 @@ template <typename R> int apply_shapes(sgpe_plan* p, int rs, int cs) {
   cudaError_t e = cudaSuccess;
   void* tx = nullptr;
   void* ty = nullptr;
-  if (rs != p->row_shape) tx = upload_twiddles<R>(p->nx, sgpe::row_points_per_thread<R>(p->nx, rs), &e);
+  const int4 *fx = nullptr, *fy = nullptr;
+  const bool fixed = p->bits == 128;
+  if (rs != p->row_shape)
+    tx = upload_twiddles<R>(p->nx, sgpe::row_points_per_thread<R>(p->nx, rs), &e, fixed ? &fx : nullptr);
   if (e == cudaSuccess && cs != p->col_shape)
-    ty = upload_twiddles<R>(p->ny, sgpe::col_points_per_thread<R>(p->ny, cs), &e);
-  void* fx = nullptr;
-  void* fy = nullptr;
-  if (p->bits == 128) {
-    if (e == cudaSuccess && tx && upload_twiddles_fx(p->nx, sgpe::row_points_per_thread<R>(p->nx, rs), &fx) != SGPE_OK)
-      e = cudaErrorMemoryAllocation;
-    if (e == cudaSuccess && ty && upload_twiddles_fx(p->ny, sgpe::col_points_per_thread<R>(p->ny, cs), &fy) != SGPE_OK)
-      e = cudaErrorMemoryAllocation;
-  }
+    ty = upload_twiddles<R>(p->ny, sgpe::col_points_per_thread<R>(p->ny, cs), &e, fixed ? &fy : nullptr);
   if (e != cudaSuccess) {
-    for (void* t : {tx, ty, fx, fy})
-      if (t) cudaFree(t);
+    if (tx) cudaFree(tx);
+    if (ty) cudaFree(ty);
     return fail(SGPE_ERR_OOM, std::string("twiddle tables: ") + cudaGetErrorString(e));
   }
   drop_graphs(p);
   // cudaFree waits for launches still reading the old tables
-  const struct { void** own; void* made; } tables[] = {{&p->tw_x, tx}, {&p->tw_y, ty}, {&p->twf_x, fx}, {&p->twf_y, fy}};
-  for (const auto& t : tables)
-    if (t.made) {
-      cudaFree(*t.own);
-      *t.own = t.made;
-    }
+  if (tx) {
+    cudaFree(p->tw_x);
+    p->tw_x = tx;
+    p->twf_x = fx;
+  }
+  if (ty) {
+    cudaFree(p->tw_y);
+    p->tw_y = ty;
+    p->twf_y = fy;
+  }
   p->row_shape = rs;
   p->col_shape = cs;
   p->ntile_fp32 = p->nx / cols;
@@ -1516,15 +1555,13 @@ int sgpe_plan_create(sgpe_plan** out, int ny, int nx, int dtype_bits, int device
   if (e == cudaSuccess) {
     by_prec(dtype_bits, [&](auto t) {
       using R = decltype(t);
-      p->tw_x = upload_twiddles<R>(nx, sgpe::row_points_per_thread<R>(nx, p->row_shape), &e);
-      if (e == cudaSuccess) p->tw_y = upload_twiddles<R>(ny, sgpe::col_points_per_thread<R>(ny, p->col_shape), &e);
+      const bool fixed = dtype_bits == 128;
+      p->tw_x = upload_twiddles<R>(nx, sgpe::row_points_per_thread<R>(nx, p->row_shape), &e, fixed ? &p->twf_x : nullptr);
+      if (e == cudaSuccess)
+        p->tw_y = upload_twiddles<R>(ny, sgpe::col_points_per_thread<R>(ny, p->col_shape), &e, fixed ? &p->twf_y : nullptr);
       return 0;
     });
   }
-  if (e == cudaSuccess && dtype_bits == 128 &&
-      (upload_twiddles_fx(nx, sgpe::row_points_per_thread<double>(nx, p->row_shape), &p->twf_x) != SGPE_OK ||
-       upload_twiddles_fx(ny, sgpe::col_points_per_thread<double>(ny, p->col_shape), &p->twf_y) != SGPE_OK))
-    e = cudaErrorMemoryAllocation;
   // the error word, and the populations that graphs write
   const size_t pops_at = 16;
   if (e == cudaSuccess)
@@ -1555,8 +1592,6 @@ int sgpe_plan_destroy(sgpe_plan* p) {
   if (p->part) cudaFree(p->part);
   if (p->tw_x) cudaFree(p->tw_x);
   if (p->tw_y) cudaFree(p->tw_y);
-  if (p->twf_x) cudaFree(p->twf_x);
-  if (p->twf_y) cudaFree(p->twf_y);
   if (p->tw64_x) cudaFree(p->tw64_x);
   if (p->tw64_y) cudaFree(p->tw64_y);
   free_sub(p->sub[0]);
@@ -1733,29 +1768,23 @@ int sgpe_set_substep(sgpe_plan* p, int sub, const sgpe_substep_ops* ops) {
   {
     const HostField ka[2] = {so.kin_host[0][0], so.kin_host[1][0]};
     const HostField kb[2] = {so.kin_host[0][1], so.kin_host[1][1]};
-    rc = build_sep_kin(p, ka, kb, &so.sep, &so.allocs);
+    FxTables fx;
+    rc = build_sep_kin(p, ka, kb, &so.sep, &so.allocs, &fx);
     HostField px[2], py[2];
     bool pot = (rc == SGPE_OK);
     for (int c = 0; c < 2 && pot; ++c)
       pot = split_xy(host_field(ops->pot_a[c]), host_field(ops->pot_b[c]), p->nx, p->ny, &px[c], &py[c]);
-    for (int c = 0; c < 2 && pot && rc == SGPE_OK; ++c) {
-      rc = upload_host_field(p, px[c], &so.sep.px[c], &so.allocs);
-      if (rc == SGPE_OK) rc = upload_host_field(p, py[c], &so.sep.py[c], &so.allocs);
-    }
-    so.sep.pot = pot && rc == SGPE_OK;
+    so.sep.pot = pot;
     HostField s01x, s10x;
     const bool cc_uniform = ops->cpl_c.sx == 0 && ops->cpl_c.sy == 0;
-    if (rc == SGPE_OK && cc_uniform && so.has_s01 && expand_1d(so.s01_host, 0, p->nx, p->ny, &s01x) &&
-        expand_1d(so.s10_host, 0, p->nx, p->ny, &s10x)) {
-      rc = upload_host_field(p, s01x, &so.sep.s01x, &so.allocs);
-      if (rc == SGPE_OK) rc = upload_host_field(p, s10x, &so.sep.s10x, &so.allocs);
-      so.sep.cpl = (rc == SGPE_OK);
-    }
+    so.sep.cpl = rc == SGPE_OK && cc_uniform && so.has_s01 && expand_1d(so.s01_host, 0, p->nx, p->ny, &s01x) &&
+                 expand_1d(so.s10_host, 0, p->nx, p->ny, &s10x);
     if (rc == SGPE_OK && so.sep.pot) {
       const HostField hc = host_field(ops->cpl_c);
       rc = build_fused(p, px, py, so.sep.cpl ? &s01x : nullptr, so.sep.cpl ? &s10x : nullptr, hc.v[0],
-                       hc.v[1], &so.sep, &so.allocs);
+                       hc.v[1], &so.sep, &so.allocs, &fx);
     }
+    if (rc == SGPE_OK) rc = fx.upload(&so.allocs);
     if (rc != SGPE_OK) {
       free_sub(so);
       return rc;
