@@ -289,3 +289,43 @@ def test_populations_on_a_captured_stream(tp, tmp_path, nx, ny):
         out.append([t.cpu().numpy() for t in p.psik] + [pops.cpu().numpy()])
     for x, y in zip(*out):
         np.testing.assert_array_equal(x, y)
+
+
+# solves of one size stepped by the grouped fixed-point kernels, next to ones
+# that keep FP64 passes (long steps; an attractive gas, whose rows alone do) and
+# one that new physics moves across that line between two calls
+@pytest.mark.parametrize('time', ['real', 'imag'])
+@pytest.mark.parametrize('side,shape', [(32, 0), (64, 0), (64, 1), (128, 2), (192, 0), (256, 2)])
+def test_grouped_batch_matches_solves_alone(tp, tmp_path, side, shape, time):
+    from spinor_gpe.batch import PropagatorBatch
+    g = (1000.0, 995.0, 990.0)
+    dt = 1e-3 if time == 'real' else 0.02
+    spins = [_problem(tmp_path / str(i), side, side, g, w) for i, w in enumerate((1.0, 0.5, None, 1.0, 0.7, 0.3))]
+    spins[4].g_sc = dict(uu=-60.0, dd=995.0, ud=300.0)
+    factor = [1.0, 1.1, 0.9, 1e4, 1.0, 1.0]    # member 3: long steps
+
+    def scaled(p, f):
+        p._plan.set_physics(*(f * p.g_sc[k] for k in ('uu', 'dd', 'ud')), float(p.atom_num),
+                            float(p._space_np['dv_r']), float(p._space_np['dv_k']), p.is_coupling)
+
+    def make():
+        out = []
+        for s, f in zip(spins, factor):
+            p = tp.TensorPropagator(s, dt, 20, 'cuda', time=time, dtype=128)
+            if shape:
+                p.kernel_shapes = (shape, shape)
+            scaled(p, f)
+            out.append(p)
+        return out
+    alone, together = make(), make()
+    batch = PropagatorBatch(together)
+    for move in (None, (5, 1e4), (3, 1.0)):
+        if move is not None:
+            for props in (alone, together):
+                scaled(props[move[0]], move[1])
+        for p in alone:
+            p.full_steps(11)
+        batch.full_steps(11)
+        for a, b in zip(alone, together):
+            np.testing.assert_array_equal([t.cpu().numpy() for t in a.psik], [t.cpu().numpy() for t in b.psik])
+    batch.close()
