@@ -412,8 +412,9 @@ int default_shape(int bits, int axis, int n) {
 // other transforms).  The pair is no faster than the large block where a wave
 // ends with both halves of most SMs taken, so the tiles of 4 are for widths
 // whose last wave fills at most half of the 304 places: us a step, 8 / 4
-// columns, nx = 256: 75.4 / 59.3, 768: 158 / 145, 2048: 317 / 305; against
-// 384: 96.0 / 100.7, 512: 92.2 / 95.2, 1024: 166.7 / 170.0.
+// columns, nx = 192: 70.1 / 54.4, 256: 69.8 / 53.5, 768: 158 / 145, 2048: 328 /
+// 315; against 384: 96.4 / 100.4, 512: 86.4 / 88.3, 1024: 166.0 / 169.6, 4096:
+// 724 / 725.
 int default_col_shape(int bits, int nx, int ny) {
   if (bits == 64 && ny == 2048) return (nx / 2) % 304 <= 152 ? 1 : 0;
   return default_shape(bits, 1, ny);

@@ -20,8 +20,11 @@
 // below 2^60.5 (its L1 norm had room), or their root sum square is below
 // 2^62.5 (that of a line whose values all add up is its largest sum).
 //
-// Precision: a product is rounded within 0.6 units and a line's values come
-// in at 2^-59 of its largest.
+// Precision: a product is rounded within 0.6 units.  A line's values come in
+// at 2^-(62 - bits(R)) of its largest, R the first radix: 2^-59 with 8 points
+// per thread, 2^-60 with 4, 2^-58 with 12 (sides 3 * 2^k).  A line whose values
+// meet in few of a stage's butterflies loses the stage's bits on the way and
+// gets them back, rounded, in front of the last stage.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -6,11 +6,12 @@
 //
 // Bound: integer issue.  At 1024^2 a column pass issues 511 instructions per
 // point and component (wide multiply-adds take their pipe for 2-2.6 cycles)
-// and a row pass 754, at two instructions per cycle and SM; DRAM and L2 are
+// and a row pass 760, at two instructions per cycle and SM; DRAM and L2 are
 // under 15% busy.  Measured at 1024^2 (real time, Raman coupling; column / row
-// / step): FP64 butterflies 347 / 473 / 2,470 us, fixed point 60.6 / 83.3 /
-// 400 us, with the error against 64 bits on average smaller (8 steps of six
-// problems, 64^2 to 4096 x 128: geometric mean 0.87 of the FP64 kernels').
+// / step): FP64 butterflies 347 / 473 / 2,470 us, fixed point 60.7 / 84.1 /
+// 403 us, with half the error against the same operations in 80 bits (90
+// problems of 2 to 20 steps, 32 x 512 to 4096 x 32: geometric mean 0.47 of the
+// FP64 kernels').
 #pragma once
 #include "sgpe_kernels.cuh"
 
